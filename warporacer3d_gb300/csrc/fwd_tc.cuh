@@ -25,10 +25,11 @@ constexpr int B_BYTES = 64 * 128;    // 64 rows x 64 bf16
 // waits return at once and no warp reads the accumulator (which no MMA may
 // have written); the results are then undefined and the error word set.
 // *issued records whether this thread issued an MMA (the drain commits only then).
+// With w1s, W1 is not resident: thread 0 copies it to OFF_W1 once layer 1 is done (w1bar).
 __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, uint32_t tmem, uint64_t* done,
                              uint32_t p0, int r, bool live, int c, int cols, float* h1g, float* h2g, float* og,
                              int write_hidden, const SampleArgs& sa, volatile int* abort, uint32_t limit,
-                             bool* issued) {
+                             bool* issued, const uint4* w1s = nullptr, uint64_t* w1bar = nullptr) {
   const int tid = threadIdx.x, warp = tid >> 5;
   bool ok = true;
   const uint32_t id64 = tc::idesc_bf16(TILE, 64), id16 = tc::idesc_bf16(TILE, 16);
@@ -38,6 +39,11 @@ __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, u
     if (!tc::mbar_wait_abort(done, p0 & 1, abort, limit)) ok = false;
     __syncwarp();  // the TMEM loads are warp-collective
     tc::tc_fence_after();
+    const bool fetch = w1s && tid == 0 && !*abort;
+    if (fetch) {  // layer 1 no longer reads W0's stages
+      tc::mbar_arrive_expect_tx(w1bar, 2 * B_BYTES);
+      tc::bulk_load(smem + OFF_W1, w1s, 2 * B_BYTES, w1bar);
+    }
     float acc[64];
     for (int layer = 0; layer < 2; ++layer) {
       if (!__any_sync(0xffffffffu, *abort != 0)) {  // warp-uniform: the loads are warp-collective
@@ -67,6 +73,7 @@ __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, u
       tc::fence_proxy_async_smem();
       tc::tc_fence_before();
       tc::named_sync(1, TILE);
+      if (layer == 0 && fetch && !tc::mbar_wait(w1bar, 0)) ok = false;
       if (tid == 0 && !*abort) {
         *issued = true;
         tc::tc_fence_after();

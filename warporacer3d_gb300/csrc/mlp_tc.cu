@@ -31,40 +31,44 @@ namespace racer {
 namespace {
 
 
-// GROUPS producer groups of four warps, one k-block in flight each (four for
-// wide inputs; two when the input has at most four k-blocks, which halves the
-// shared memory so two CTAs share an SM), plus one MMA warp.
-template <int GROUPS>
+// Two producer groups of four warps, one k-block in flight each in registers
+// (64 KB of loads an SM, 128 KB with two CTAs), plus one MMA warp. Shared
+// memory is kept to 54 KB: the SM's L1 is what its resident CTAs leave of 256
+// KB, and the lidar of another rollout chain or stream that shares the SM
+// gathers its cells through it (k_lidar_track at 4096 cars x 1081 beams takes
+// 119 us with 224 KB of L1, 122 with 118 KB, 133 with 28 KB). So W1 takes the
+// place of W0's stages once layer 1 is done (a bulk copy behind the first
+// tanh), and no stage is deeper than the loads in flight need. The TMA-staged
+// kernel below (200 KB) in this place made a 64-step rollout of 4096 cars in
+// 16 chains 7.12 ms against 6.45.
 struct FwdCfg {
+  static constexpr int GROUPS = 2;
   static constexpr int THREADS = (GROUPS * 4 + 1) * 32;
   static constexpr int MMA_WARP = GROUPS * 4;
   static constexpr int OFF_A = 0;  // GROUPS x A; H = [h | 1 | 0] reuses A[0], A[1]
   static constexpr int OFF_B = OFF_A + GROUPS * A_BYTES;
-  static constexpr int OFF_W1 = OFF_B + GROUPS * B_BYTES;
-  static constexpr int OFF_W2 = OFF_W1 + 2 * B_BYTES;
+  static constexpr int OFF_W1 = OFF_B;  // takes the place of W0's stages once layer 1 is done
+  static constexpr int OFF_W2 = OFF_B + GROUPS * B_BYTES;
   static constexpr int OFF_BAR = OFF_W2 + 2 * 16 * 128;
-  // + barriers, + alignment slack, + 16 KB so every descriptor-addressed read stays inside the allocation
-  static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024 + 16384;
-  static constexpr int MIN_BLOCKS = GROUPS == 2 ? 2 : 1;
-  static_assert((2 * GROUPS + 3) * 8 + 8 <= 128, "barriers, the TMEM slot and the abort word fit their 128 bytes");
+  static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;  // + barriers, + alignment slack
+  static_assert((2 * GROUPS + 4) * 8 + 8 <= 128, "barriers, the TMEM slot and the abort word fit their 128 bytes");
 };
 
 
-// Grid: one CTA per 128 samples. Warps 0-15 form four producer groups; group
-// g loads k-blocks g, g+4, g+8, ... of X (thread = sample row) and of W0 into
-// stage g, then arrives on full[g]. Warp 16 waits on full[kb % 4], issues the
-// four K=16 MMAs of the block and commits to empty[kb % 4]; after the last
+// Grid: one CTA per 128 samples. Warps 0-7 form two producer groups; group
+// g loads k-blocks g, g+2, g+4, ... of X (thread = sample row) and of W0 into
+// stage g, then arrives on full[g]. Warp 8 waits on full[kb % 2], issues the
+// four K=16 MMAs of the block and commits to empty[kb % 2]; after the last
 // block it commits to `done`. Warps 0-3 (TMEM lanes 0-127) then run the
 // epilogues and issue layers 2 and 3.
-template <int GROUPS>
-__global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, FwdCfg<GROUPS>::MIN_BLOCKS)
+__global__ void __launch_bounds__(FwdCfg::THREADS, 2)
     k_mlp_fwd(const float* __restrict__ x, int in, int cols, int c0, int c1,
                                                         const uint4* __restrict__ w0s, int kblocks,
                                                         const uint4* __restrict__ w1s,
                                                         const uint4* __restrict__ w2s, float* h1g, float* h2g,
                                                         float* og, int write_hidden, SampleArgs sa, int* err) {
-  using C = FwdCfg<GROUPS>;
-  constexpr int THREADS = C::THREADS, MMA_WARP = C::MMA_WARP, OFF_A = C::OFF_A, OFF_B = C::OFF_B,
+  using C = FwdCfg;
+  constexpr int GROUPS = C::GROUPS, THREADS = C::THREADS, MMA_WARP = C::MMA_WARP, OFF_A = C::OFF_A, OFF_B = C::OFF_B,
                 OFF_W1 = C::OFF_W1, OFF_W2 = C::OFF_W2, OFF_BAR = C::OFF_BAR;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = tc::smem_u32(smem_raw);
@@ -73,7 +77,8 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, FwdCfg<GROUPS>::MIN_B
   uint64_t* empty = full + GROUPS;
   uint64_t* done = empty + GROUPS;
   uint64_t* drain = done + 1;  // [2]: thread 0's and the MMA lane's final commits after a timeout
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(drain + 2);
+  uint64_t* w1bar = drain + 2;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(w1bar + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tslot + 1);  // set by a timed-out wait
   constexpr uint32_t limit = tc::WAIT_LIMIT;
 
@@ -88,6 +93,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, FwdCfg<GROUPS>::MIN_B
       tc::mbar_init(&empty[g], 1);
     }
     tc::mbar_init(done, 1);
+    tc::mbar_init(w1bar, 1);
     tc::mbar_init(&drain[0], 1);
     tc::mbar_init(&drain[1], 1);
     *abort = 0;
@@ -98,9 +104,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, FwdCfg<GROUPS>::MIN_B
     tc::tmem_relinquish();
   }
   {  // W1 (2 x 8 KB) and W2 (2 x 2 KB), resident for the whole tile
-    uint4* w1 = reinterpret_cast<uint4*>(smem + OFF_W1);
     uint4* w2 = reinterpret_cast<uint4*>(smem + OFF_W2);
-    for (int e = tid; e < 2 * B_BYTES / 16; e += THREADS) w1[e] = __ldg(w1s + e);
     for (int e = tid; e < 2 * 16 * 128 / 16; e += THREADS) w2[e] = __ldg(w2s + e);
   }
   tc::fence_proxy_async_smem();
@@ -160,7 +164,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, FwdCfg<GROUPS>::MIN_B
   }
 
   if (warp < 4 && !fwd_epilogue(smem, OFF_A, OFF_W1, OFF_W2, tmem, done, 0, r, live, c, cols, h1g, h2g, og,
-                                  write_hidden, sa, abort, limit, &issued))
+                                  write_hidden, sa, abort, limit, &issued, w1s, w1bar))
     ok = false;
   tc::tc_fence_before();
   __syncthreads();
@@ -189,7 +193,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, FwdCfg<GROUPS>::MIN_B
 // Features past `in` and samples past `cols` read zero, as the register
 // path's loads do; samples of a box outside [c0, c1) are never written back.
 // The epilogues are the register path's, so both give the same bits.
-// PERSIST: CTA b takes tiles b, b + gridDim.x, ...; the rings' stages and
+// CTA b takes tiles b, b + gridDim.x, ...; the rings' stages and
 // parities run on across tiles, so the TMA warp loads the next tile's first
 // boxes while warps 0-3 run this tile's epilogue. Layer 1 of the next tile
 // starts only after those warps packed its first k-block, which follows their
@@ -210,7 +214,6 @@ struct TmaCfg {
 static_assert(TmaCfg::SMEM_BYTES <= 227 * 1024, "one CTA per SM");
 static_assert((2 * XS + 2 * XA + 3) * 8 + 8 <= 256, "barriers, the TMEM slot and the abort word fit their 256 bytes");
 
-template <bool PERSIST>
 __global__ void __launch_bounds__(TmaCfg::THREADS, 1)
     k_mlp_fwd_tma(const __grid_constant__ CUtensorMap xmap, int cols, int c0, int c1, const uint4* __restrict__ w0s,
                   int kblocks, const uint4* __restrict__ w1s, const uint4* __restrict__ w2s, float* h1g, float* h2g,
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(TmaCfg::THREADS, 1)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r = tid & (TILE - 1);
   const int tiles = (c1 - c0 + TILE - 1) / TILE;
-  const int stride = PERSIST ? (int)gridDim.x : tiles;  // one tile per CTA unless persistent
+  const int stride = (int)gridDim.x;
 
   if (tid == 0) {
     for (int s = 0; s < XS; ++s) {
@@ -442,18 +445,17 @@ void launch_pack_weights(const float* theta, int in, uint8_t* pack, cudaStream_t
   k_pack_weights<<<device_sms(), 256, 0, st>>>(theta, in, kb, w0, w1, w2);
 }
 
-template <int GROUPS>
 static cudaError_t fwd_launch(const float* x, int in, int cols, int c0, int c1, int kb, const uint4* w0,
                               const uint4* w1, const uint4* w2, float* h1, float* h2, float* o, int write_hidden,
                               const SampleArgs& sa, int* err, cudaStream_t st) {
-  using C = FwdCfg<GROUPS>;
+  using C = FwdCfg;
   static unsigned long long configured = 0;  // per device
   cudaError_t e = once_per_device(&configured, [] {
-    return cudaFuncSetAttribute(k_mlp_fwd<GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    return cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
   });
   if (e != cudaSuccess) return e;
   if (c1 <= c0) return cudaSuccess;
-  k_mlp_fwd<GROUPS><<<(c1 - c0 + TILE - 1) / TILE, C::THREADS, C::SMEM_BYTES, st>>>(x, in, cols, c0, c1, w0, kb, w1, w2,
+  k_mlp_fwd<<<(c1 - c0 + TILE - 1) / TILE, C::THREADS, C::SMEM_BYTES, st>>>(x, in, cols, c0, c1, w0, kb, w1, w2,
                                                                                   h1, h2, o, write_hidden, sa, err);
   return cudaGetLastError();
 }
@@ -465,32 +467,26 @@ cudaError_t launch_mlp_fwd(const float* x, int in, int cols, const uint8_t* pack
   const uint4* w0 = reinterpret_cast<const uint4*>(pack);
   const uint4* w1 = reinterpret_cast<const uint4*>(pack + (size_t)kb * 8192);
   const uint4* w2 = reinterpret_cast<const uint4*>(pack + (size_t)kb * 8192 + 2 * 8192);
-  if (kb <= 4) return fwd_launch<2>(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
-  // wide inputs: X staged by TMA where its sample columns are 16-byte aligned
+  const int sms = device_sms(), tiles = (c1 - c0 + TILE - 1) / TILE;
+  // Wide inputs with more 128-sample tiles than SMs and 16-byte aligned sample columns: one
+  // persistent CTA per SM, each running ahead into its next tile (65536 cars, 1086 inputs: 72 us;
+  // without that alignment 40001 cars took 60 us in the register-staged kernel). With no more
+  // tiles than SMs a CTA has one tile; its TMA-staged form is the faster by itself (4096 cars: 18 us
+  // against 22), but the small kernel leaves the SM its L1 (FwdCfg).
   CUtensorMap xmap;
-  if (c1 > c0 && (cols & 3) == 0 && (c0 & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
+  if (kb > 4 && sms > 0 && tiles > sms && (cols & 3) == 0 && (c0 & 3) == 0 &&
+      (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
       make_tmap_f32(&xmap, x, (uint64_t)in, (uint64_t)cols, (uint64_t)cols, TILE, 64) == 0) {
     static unsigned long long configured = 0;  // per device
     cudaError_t e = once_per_device(&configured, [] {
-      for (auto* k : {k_mlp_fwd_tma<false>, k_mlp_fwd_tma<true>}) {
-        cudaError_t a = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TmaCfg::SMEM_BYTES);
-        if (a != cudaSuccess) return a;
-      }
-      return cudaSuccess;
+      return cudaFuncSetAttribute(k_mlp_fwd_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, TmaCfg::SMEM_BYTES);
     });
     if (e != cudaSuccess) return e;
-    const int sms = device_sms();
-    // more tiles than SMs: one persistent CTA per SM, each running ahead into its next tile
-    const int tiles = (c1 - c0 + TILE - 1) / TILE;
-    if (sms > 0 && tiles > sms)
-      k_mlp_fwd_tma<true><<<sms, TmaCfg::THREADS, TmaCfg::SMEM_BYTES, st>>>(xmap, cols, c0, c1, w0, kb, w1, w2, h1, h2,
-                                                                           o, write_hidden, sa, err);
-    else
-      k_mlp_fwd_tma<false><<<tiles, TmaCfg::THREADS, TmaCfg::SMEM_BYTES, st>>>(xmap, cols, c0, c1, w0, kb, w1, w2, h1,
-                                                                             h2, o, write_hidden, sa, err);
+    k_mlp_fwd_tma<<<sms, TmaCfg::THREADS, TmaCfg::SMEM_BYTES, st>>>(xmap, cols, c0, c1, w0, kb, w1, w2, h1, h2, o,
+                                                                   write_hidden, sa, err);
     return cudaGetLastError();
   }
-  return fwd_launch<4>(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
+  return fwd_launch(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
 }
 
 }  // namespace racer

@@ -887,20 +887,39 @@ static LidarGrid lidar_grid(const Segments& g, const LidarShape& shape) {
   return lg;
 }
 
+// A lidar grid of at least BIG_LIDAR blocks asks for SMs whose shared memory is
+// the 32 KB that 32 resident blocks reserve, the rest of the 256 KB being L1. An
+// SM keeps the split of the last kernel that needed more (a policy forward or a
+// learned lidar of another stream) until it drains, which under a long lidar it
+// does not: with 28 KB of L1 the step of 119,808 cars on five tracks takes
+// 7.2 ms, with this 6.1. The switch waits for the SM to drain, so small grids do
+// without (4352 blocks, one of 16 rollout chains: 6.45 ms a rollout against 6.88).
+constexpr long BIG_LIDAR = 1 << 18;
+template <class... P, class... A>
+static void lidar_launch(void (*k)(P...), dim3 grid, unsigned threads, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at.val.sharedMemCarveout = 14;  // per cent of 228 KB
+  cfg.attrs = &at, cfg.numAttrs = (long)grid.x * grid.y >= BIG_LIDAR ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 template <int LAYERS, int CARS, bool WIDE>
 static void lidar_track(const TrackDev& t, int max_iters, const float4* ray, float* obs, int n, int c0, int c1,
                         int beams, const float2* beam_dir, int* iters, cudaStream_t st, bool flat = false) {
   const long items = (long)(c1 - c0) * beams;
   if (flat && items > 0 && items < (1L << 31)) {
     const unsigned blocks = (unsigned)((items + 32 * CARS - 1) / (32 * CARS));
-    k_lidar_flat<LAYERS, CARS, WIDE><<<blocks, CARS * 32, 0, st>>>(t, max_iters, ray, obs, n, c0, (unsigned)items,
-                                                                   beams, beam_dir, iters);
+    lidar_launch(k_lidar_flat<LAYERS, CARS, WIDE>, dim3(blocks), CARS * 32, st, t, max_iters, ray, obs, n, c0,
+                 (unsigned)items, beams, beam_dir, iters);
     return;
   }
   dim3 grid((c1 - c0 + CARS - 1) / CARS, (beams + 31) / 32);
   if (grid.x == 0) return;
-  k_lidar_track<LAYERS, CARS, WIDE, false>
-      <<<grid, CARS * 32, 0, st>>>(t, max_iters, ray, obs, n, c0, c1, beams, beam_dir, iters, nullptr, nullptr);
+  lidar_launch(k_lidar_track<LAYERS, CARS, WIDE, false>, grid, CARS * 32, st, t, max_iters, ray, obs, n, c0, c1, beams,
+               beam_dir, iters, (const int*)nullptr, (const int*)nullptr);
 }
 
 template <int LAYERS, bool WIDE>
@@ -948,7 +967,7 @@ static void lidar_shape(const Segments& g, const LidarShape& shape, const float4
   }
   const LidarGrid lg = lidar_grid(g, shape);
   dim3 grid(lg.block0[g.count], (beams + 31) / 32);
-  k_lidar_segments<CARS, WIDE><<<grid, CARS * 32, 0, st>>>(g, lg, ray, obs, n, beams, beam_dir, iters);
+  lidar_launch(k_lidar_segments<CARS, WIDE>, grid, CARS * 32, st, g, lg, ray, obs, n, beams, beam_dir, iters);
 }
 
 bool lidar_shape_ok(const LidarShape& shape) {
