@@ -71,22 +71,25 @@ RM_HD float cos_kernel(float r2) {
 // quadrant |k| = rint(|x| 2/pi) <= 4092 < 2^12, where k * PIO2_A and
 // k * PIO2_B are exact: beyond it the reduction would lose bits silently.
 #define RM_SINCOS_MAX 6426.0f
+// The quadrant picks by swaps and sign flips, not by branches: neighbouring
+// cars' headings lie in different quadrants, and a warp would run each case.
+// sincos_in holds for |x| <= RM_SINCOS_MAX only.
+RM_HD void sincos_in(float x, float* s, float* c) {
+  float kf = rintf(x * RM_TWO_OVER_PI);
+  uint32_t k = (uint32_t)(int)kf;
+  float r = ((x - kf * RM_PIO2_A) - kf * RM_PIO2_B) - kf * RM_PIO2_C;
+  float r2 = r * r;
+  float sr = sin_kernel(r, r2), cr = cos_kernel(r2);
+  float a = (k & 1u) ? cr : sr, b = (k & 1u) ? sr : cr;
+  *s = from_bits(to_bits(a) ^ ((k & 2u) << 30));
+  *c = from_bits(to_bits(b) ^ (((k + 1u) & 2u) << 30));
+}
 RM_HD void sincosf_(float x, float* s, float* c) {
   if (!(fabsf(x) <= RM_SINCOS_MAX)) {
     *s = *c = x - x + from_bits(0x7fc00000u);
     return;
   }
-  float kf = rintf(x * RM_TWO_OVER_PI);
-  int k = (int)kf;
-  float r = ((x - kf * RM_PIO2_A) - kf * RM_PIO2_B) - kf * RM_PIO2_C;
-  float r2 = r * r;
-  float sr = sin_kernel(r, r2), cr = cos_kernel(r2);
-  switch (k & 3) {
-    case 0: *s = sr; *c = cr; break;
-    case 1: *s = cr; *c = -sr; break;
-    case 2: *s = -sr; *c = -cr; break;
-    default: *s = -cr; *c = sr; break;
-  }
+  sincos_in(x, s, c);
 }
 RM_HD float sinf_(float x) { float s, c; sincosf_(x, &s, &c); return s; }
 RM_HD float cosf_(float x) { float s, c; sincosf_(x, &s, &c); return c; }

@@ -20,6 +20,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "exact.cuh"
 #include "fwd_tc.cuh"
 #include "kernels.h"
 #include "philox.h"
@@ -32,6 +33,7 @@ namespace {
 struct Spot {
   int layer;
   float clearance, height;
+  int cell;  // index of the probed cell, -1 off the map
 };
 struct Surface {
   float height, sx, sy;
@@ -39,11 +41,17 @@ struct Surface {
 
 __device__ __forceinline__ float clampf_(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 
-__device__ __forceinline__ void slopes(const Surface& g, float heading, float* along, float* across) {
+template <class M>
+__device__ __forceinline__ void slopes(M& m, const Surface& g, float heading, float* along, float* across) {
   float s, c;
-  rmath::sincosf_(heading, &s, &c);
+  m.sincos(heading, &s, &c);
   *along = g.sx * c + g.sy * s;
   *across = -g.sx * s + g.sy * c;
+}
+
+__device__ __forceinline__ void slopes(const Surface& g, float heading, float* along, float* across) {
+  Ieee m;
+  slopes(m, g, heading, along, across);
 }
 
 // floor((v - v0) / cell + 0.5), the reference's nearest-cell coordinate
@@ -133,40 +141,57 @@ __device__ __forceinline__ unsigned lidar_cell(const TrackDev& t, float vx, floa
   return min(iy, (unsigned)t.ny) * (unsigned)t.lw + min(ix, (unsigned)t.nx);
 }
 
-// racer/sim.mojo:116-124. LAYERS = 0 reads the layer count from the track.
-// The first drivable layer is taken only if |height - z| < 1e30 (the initial
-// gap). GUARD = false drops that test where it cannot fail: grid heights are
-// finite with |h| <= 1e6 (checked on upload) and the caller knows |z| <= 1e20
-// + 10, so the result is the same.
+// racer/sim.mojo:116-124 on a cell's (clearance, height) of its one or two
+// layers. The first drivable layer is taken only if |height - z| < 1e30 (the
+// initial gap). GUARD = false drops that test where it cannot fail: grid
+// heights are finite with |h| <= 1e6 (checked on upload) and the caller knows
+// |z| <= 1e20 + 10, so the result is the same.
+template <bool GUARD>
+__device__ __forceinline__ Spot pick(float4 v, int cell, float z) {
+  Spot best{0, -1.0f, v.y, cell};
+  float gap = 1e30f;
+  if (v.x > 0.0f && (!GUARD || fabsf(v.y - z) < gap)) {
+    best.clearance = v.x;
+    gap = fabsf(v.y - z);
+  }
+  if (v.z > 0.0f && fabsf(v.w - z) < gap) best = Spot{1, v.z, v.w, cell};
+  return best;
+}
+template <bool GUARD>
+__device__ __forceinline__ Spot pick(float2 v, int cell, float z) {
+  return Spot{0, v.x > 0.0f && (!GUARD || fabsf(v.y - z) < 1e30f) ? v.x : -1.0f, v.y, cell};
+}
+
+// The cell k of the repacked grid of one or two layers.
+template <int LAYERS>
+struct CellOf {
+  using type = float2;
+};
+template <>
+struct CellOf<2> {
+  using type = float4;
+};
+template <int LAYERS>
+__device__ __forceinline__ typename CellOf<LAYERS>::type load_cell(const TrackDev& t, long k) {
+  return __ldg(reinterpret_cast<const typename CellOf<LAYERS>::type*>(t.cl) + k);
+}
+
+// LAYERS = 0 reads the layer count from the track.
 template <int LAYERS, bool GUARD = true>
 __device__ __forceinline__ Spot probe(const TrackDev& t, float x, float y, float z) {
   long idx;
-  if (!cell_of(t, x, y, &idx)) return Spot{0, -1.0f, -1.0f};  // off the map every grid reads -1
-  Spot best;
+  if (!cell_of(t, x, y, &idx)) return Spot{0, -1.0f, -1.0f, -1};  // off the map every grid reads -1
+  if (LAYERS == 1 || LAYERS == 2) return pick<GUARD>(load_cell<LAYERS>(t, idx), (int)idx, z);
+  const int L = t.layers;
+  const float2* p = t.cl + idx * L;
+  float2 v0 = __ldg(p);
+  Spot best{0, -1.0f, v0.y, (int)idx};
   float gap = 1e30f;
-  if (LAYERS == 2) {
-    float4 v = __ldg(reinterpret_cast<const float4*>(t.cl) + idx);
-    best = Spot{0, -1.0f, v.y};
-    if (v.x > 0.0f && (!GUARD || fabsf(v.y - z) < gap)) {
-      best = Spot{0, v.x, v.y};
+  for (int l = 0; l < L; ++l) {
+    float2 v = __ldg(p + l);
+    if (v.x > 0.0f && fabsf(v.y - z) < gap) {
+      best = Spot{l, v.x, v.y, (int)idx};
       gap = fabsf(v.y - z);
-    }
-    if (v.z > 0.0f && fabsf(v.w - z) < gap) best = Spot{1, v.z, v.w};
-  } else if (LAYERS == 1) {
-    float2 v = __ldg(t.cl + idx);
-    best = Spot{0, -1.0f, v.y};
-    if (v.x > 0.0f && (!GUARD || fabsf(v.y - z) < gap)) best = Spot{0, v.x, v.y};
-  } else {
-    const int L = t.layers;
-    const float2* p = t.cl + idx * L;
-    float2 v0 = __ldg(p);
-    best = Spot{0, -1.0f, v0.y};
-    for (int l = 0; l < L; ++l) {
-      float2 v = __ldg(p + l);
-      if (v.x > 0.0f && fabsf(v.y - z) < gap) {
-        best = Spot{l, v.x, v.y};
-        gap = fabsf(v.y - z);
-      }
     }
   }
   return best;
@@ -203,9 +228,12 @@ struct SurfaceCell {
   float tx, ty;
 };
 
-__device__ __forceinline__ SurfaceCell surface_cell(const TrackDev& t, float x, float y) {
-  float fx = (x - t.x0) / t.cell;
-  float fy = (y - t.y0) / t.cell;
+template <class M>
+__device__ __forceinline__ SurfaceCell surface_cell(M& m, const TrackDev& t, float x, float y) {
+  const float dx = x - t.x0, dy = y - t.y0;
+  m.need((t.cell >= B_MIN) & (t.cell <= B_MAX));
+  float fx = m.div(dx, t.cell, t.inv_cell);
+  float fy = m.div(dy, t.cell, t.inv_cell);
   float flx = floorf(fx), fly = floorf(fy);
   int ix = flx >= 0.0f ? (flx <= (float)(t.nx - 2) ? (int)flx : t.nx - 2) : 0;
   int iy = fly >= 0.0f ? (fly <= (float)(t.ny - 2) ? (int)fly : t.ny - 2) : 0;
@@ -217,46 +245,86 @@ __device__ __forceinline__ float4 surface_corners(const TrackDev& t, int layer, 
   return make_float4(__ldg(hp), __ldg(hp + 1), __ldg(hp + t.nx), __ldg(hp + t.nx + 1));
 }
 
-__device__ __forceinline__ Surface surface_blend(const TrackDev& t, const SurfaceCell& c, float4 h) {
+template <class M>
+__device__ __forceinline__ Surface surface_blend(M& m, const TrackDev& t, const SurfaceCell& c, float4 h) {
   const float tx = c.tx, ty = c.ty;
   float w0 = (1.0f - tx) * (1.0f - ty), w1 = tx * (1.0f - ty), w2 = (1.0f - tx) * ty, w3 = tx * ty;
   Surface s;
   s.height = (h.x * w0 + h.z * w2) + (h.y * w1 + h.w * w3);
-  s.sx = ((h.y - h.x) * (1.0f - ty) + (h.w - h.z) * ty) / t.cell;
-  s.sy = ((h.z - h.x) * (1.0f - tx) + (h.w - h.y) * tx) / t.cell;
+  s.sx = m.div((h.y - h.x) * (1.0f - ty) + (h.w - h.z) * ty, t.cell, t.inv_cell);
+  s.sy = m.div((h.z - h.x) * (1.0f - tx) + (h.w - h.y) * tx, t.cell, t.inv_cell);
   return s;
 }
 
 __device__ __forceinline__ Surface surface(const TrackDev& t, int layer, float x, float y) {
-  const SurfaceCell c = surface_cell(t, x, y);
-  return surface_blend(t, c, surface_corners(t, layer, c.base));
+  Ieee m;
+  const SurfaceCell c = surface_cell(m, t, x, y);
+  return surface_blend(m, t, c, surface_corners(t, layer, c.base));
 }
 
-// Probe and the surface under the chosen layer. With two layers the corner
-// heights of both layers are loaded alongside the probe and those of the
-// chosen layer blended, so the loads do not wait for the layer.
+// Loads a line into L1 that a later load of this thread will want; nothing waits for it.
+__device__ __forceinline__ void touch(const void* p) {
+  asm volatile("{\n .reg .f32 v;\n ld.global.nc.f32 v, [%0];\n}\n" ::"l"(p));
+}
+
+__device__ __forceinline__ float4 heights(float4 a, float4 b, float4 c, float4 d, int layer) {
+  return layer ? make_float4(a.w, b.w, c.w, d.w) : make_float4(a.y, b.y, c.y, d.y);
+}
+__device__ __forceinline__ float4 heights(float2 a, float2 b, float2 c, float2 d, int) {
+  return make_float4(a.y, b.y, c.y, d.y);
+}
+
+// Probe and the surface under the chosen layer. With one or two layers the
+// corners come from the repacked cells (the same heights), which hold every
+// layer and the probed cell itself: five loads from two rows, none waiting for
+// the layer, where the layers' own height grids took nine from five. The 32
+// cars of a warp are in 32 places, so a load costs the warp a line per car.
+// The rows a car may enter in its next substep (it moves less than a cell) are
+// fetched meanwhile: without that some car of the warp misses L1 every time.
+template <int LAYERS, class M>
+__device__ __forceinline__ Surface probe_surface(M& m, const TrackDev& t, float x, float y, float z, Spot* spot) {
+  const SurfaceCell c = surface_cell(m, t, x, y);
+  if (LAYERS == 0) {
+    *spot = probe<LAYERS>(t, x, y, z);
+    return surface_blend(m, t, c, surface_corners(t, spot->layer, c.base));
+  }
+  const auto a = load_cell<LAYERS>(t, c.base), b = load_cell<LAYERS>(t, c.base + 1),
+             d = load_cell<LAYERS>(t, c.base + t.nx), e = load_cell<LAYERS>(t, c.base + t.nx + 1);
+  *spot = probe<LAYERS>(t, x, y, z);
+  return surface_blend(m, t, c, heights(a, b, d, e, spot->layer));
+}
+
+// The rows before and after the probed cell's, in L1 for the next substep's probe.
+template <int LAYERS>
+__device__ __forceinline__ void touch_rows(const TrackDev& t, int cell) {
+  if (LAYERS == 0 || cell < 0) return;
+  const long last = (long)t.nx * t.ny - 1;
+  touch(t.cl + max((long)cell - t.nx, 0l) * LAYERS);
+  touch(t.cl + min((long)cell + t.nx, last) * LAYERS);
+}
+
 template <int LAYERS>
 __device__ __forceinline__ Surface probe_surface(const TrackDev& t, float x, float y, float z, Spot* spot) {
-  if (LAYERS == 2) {
-    const SurfaceCell c = surface_cell(t, x, y);
-    const float4 h0 = surface_corners(t, 0, c.base), h1 = surface_corners(t, 1, c.base);
-    *spot = probe<LAYERS>(t, x, y, z);
-    return surface_blend(t, c, spot->layer ? h1 : h0);
-  }
-  *spot = probe<LAYERS>(t, x, y, z);
-  return surface(t, spot->layer, x, y);
+  Chain m;
+  const Surface s = probe_surface<LAYERS>(m, t, x, y, z, spot);
+  if (m.ok) return s;
+  Ieee e;
+  return probe_surface<LAYERS>(e, t, x, y, z, spot);
 }
 
 __device__ __forceinline__ float waypoint(const TrackDev& t, long w, int field) {
   return __ldg(t.d + t.route + 4 * w + field);
 }
 
-// racer/sim.mojo:146-152. Off the map the nearest grid reads -1 and the
-// route lookup lands on d[route - 4 + field], as in the reference.
-__device__ __forceinline__ float progress(const TrackDev& t, int layer, float x, float y) {
-  long idx;
-  long w = -1;
-  if (cell_of(t, x, y, &idx)) w = (long)__ldg(t.d + HEADER + (long)(3 * layer + 2) * t.nx * t.ny + idx);
+// racer/sim.mojo:146-152 at the cell of the last probe (-1 off the map).
+// Off the map the nearest grid reads -1 and the route lookup lands on
+// d[route - 4 + field], as in the reference.
+__device__ __forceinline__ long nearest(const TrackDev& t, int layer, int cell) {
+  return cell < 0 ? -1 : (long)__ldg(t.d + HEADER + (long)(3 * layer + 2) * t.nx * t.ny + cell);
+}
+
+__device__ __forceinline__ float progress(const TrackDev& t, int layer, int cell, float x, float y) {
+  const long w = nearest(t, layer, cell);
   float heading = waypoint(t, w, 3);
   float s, c;
   rmath::sincosf_(heading, &s, &c);
@@ -268,26 +336,59 @@ struct V4 {
   float x, y, h, s;  // position, heading, speed
 };
 
-// racer/sim.mojo:155-167
-__device__ __forceinline__ V4 derivative(const V4& p, float steer, float accel, float grip, float along,
-                                         float across) {
-  float nz = 1.0f / sqrtf((1.0f + along * along) + across * across);
-  float load = (grip * GRAV) * nz;
-  float v = fmaxf(fabsf(p.s), 0.5f) * (p.s >= 0.0f ? 1.0f : -1.0f);
-  float slide = (GRAV * across) * nz;
-  float ss, cs;
-  rmath::sincosf_(steer, &ss, &cs);
-  float lateral = clampf_((((v * p.s) * ss) / cs) / WHEELBASE + slide, -load, load);
-  float yaw = (lateral - slide) / v;
-  float longitudinal = sqrtf(fmaxf(load * load - lateral * lateral, 0.0f));
-  float dv = clampf_(accel, -longitudinal, longitudinal) - (GRAV * along) * nz;
+// What a derivative takes from the steering angle alone, known before the stages that use it.
+struct Steer {
+  float s, c, rc;  // sine, cosine, RN(1 / cosine)
+};
+template <class M>
+__device__ __forceinline__ Steer steer_terms(M& m, float steer) {
+  Steer q;
+  m.sincos(steer, &q.s, &q.c);
+  q.rc = m.rcp(q.c);
+  return q;
+}
+
+// racer/sim.mojo:155-167, the terms of the ground (nz, load, slide, once per substep) and of the steering given.
+template <class M>
+__device__ __forceinline__ V4 derivative(M& m, const V4& p, const Steer& st, float accel, float nz, float load,
+                                         float slide, float along) {
+  const float v = fmaxf(fabsf(p.s), 0.5f) * (p.s >= 0.0f ? 1.0f : -1.0f);
+  const float rv = m.rcp(v);
+  const float turn = m.div(m.div((v * p.s) * st.s, st.c, st.rc), WHEELBASE, 1.0f / WHEELBASE);
+  const float lateral = clampf_(turn + slide, -load, load);
+  const float yaw = m.div(lateral - slide, v, rv);
+  const float longitudinal = m.root(fmaxf(load * load - lateral * lateral, 0.0f));
+  const float dv = clampf_(accel, -longitudinal, longitudinal) - (GRAV * along) * nz;
   float sh, ch;
-  rmath::sincosf_(p.h, &sh, &ch);
+  m.sincos(p.h, &sh, &ch);
   return V4{p.s * ch, p.s * sh, yaw, dv};
 }
 
 __device__ __forceinline__ V4 axpy(const V4& p, const V4& k, float h) {
   return V4{p.x + k.x * h, p.y + k.y * h, p.h + k.h * h, p.s + k.s * h};
+}
+
+// One RK4 substep (racer/sim.mojo:197-209) from p on `ground`, before the speed's clamp.
+template <class M>
+__device__ __forceinline__ V4 rk4(M& m, V4 p, const Surface& ground, float steer, float rate, float accel, float grip) {
+  const float half_dt = DT / 2.0f, sixth_dt = DT / 6.0f;
+  float along, across;
+  slopes(m, ground, p.h, &along, &across);
+  const float norm2 = (1.0f + along * along) + across * across;
+  const float nz = m.rcp(m.root(norm2));
+  const float load = (grip * GRAV) * nz, slide = (GRAV * across) * nz;
+  m.need((norm2 <= A_MAX) & (fabsf(load) <= 1.12589991e+15f));  // 2^50: |lateral| <= |load| bounds the root's operand
+  const Steer start = steer_terms(m, steer), mid = steer_terms(m, steer + (rate * DT) / 2.0f),
+              end = steer_terms(m, steer + rate * DT);
+  const V4 k1 = derivative(m, p, start, accel, nz, load, slide, along);
+  const V4 k2 = derivative(m, axpy(p, k1, half_dt), mid, accel, nz, load, slide, along);
+  const V4 k3 = derivative(m, axpy(p, k2, half_dt), mid, accel, nz, load, slide, along);
+  const V4 k4 = derivative(m, axpy(p, k3, DT), end, accel, nz, load, slide, along);
+  p.x = p.x + ((k1.x + 2.0f * (k2.x + k3.x)) + k4.x) * sixth_dt;
+  p.y = p.y + ((k1.y + 2.0f * (k2.y + k3.y)) + k4.y) * sixth_dt;
+  p.h = p.h + ((k1.h + 2.0f * (k2.h + k3.h)) + k4.h) * sixth_dt;
+  p.s = p.s + ((k1.s + 2.0f * (k2.s + k3.s)) + k4.s) * sixth_dt;
+  return p;
 }
 
 // racer/sim.mojo:170-181. `local` is the car's index within its track's
@@ -338,34 +439,38 @@ __device__ __forceinline__ void advance_car(const TrackDev& t, float* s, const f
   float rate = clampf_(act[i], -1.0f, 1.0f) * STEER_RATE;
   float accel = clampf_(act[(long)n + i], -1.0f, 1.0f) * ACCEL_MAX;
   float grip = GRIP * s[(long)FRICTION * n + i];
+  const float progress0 = s[(long)PROGRESS * n + i], steps0 = s[(long)STEPS * n + i], return0 = s[(long)RETURN * n + i];
   bool crashed = false;
-  const float half_dt = DT / 2.0f, sixth_dt = DT / 6.0f;
+  touch_rows<LAYERS>(t, spot.cell);
 #pragma unroll 1
   for (int sub = 0; sub < SUBSTEPS; ++sub) {
-    float along, across;
-    slopes(ground, p.h, &along, &across);
-    float mid = steer + (rate * DT) / 2.0f;
-    V4 k1 = derivative(p, steer, accel, grip, along, across);
-    V4 k2 = derivative(axpy(p, k1, half_dt), mid, accel, grip, along, across);
-    V4 k3 = derivative(axpy(p, k2, half_dt), mid, accel, grip, along, across);
-    V4 k4 = derivative(axpy(p, k3, DT), steer + rate * DT, accel, grip, along, across);
-    p.x = p.x + ((k1.x + 2.0f * (k2.x + k3.x)) + k4.x) * sixth_dt;
-    p.y = p.y + ((k1.y + 2.0f * (k2.y + k3.y)) + k4.y) * sixth_dt;
-    p.h = p.h + ((k1.h + 2.0f * (k2.h + k3.h)) + k4.h) * sixth_dt;
-    p.s = p.s + ((k1.s + 2.0f * (k2.s + k3.s)) + k4.s) * sixth_dt;
+    Chain m;
+    V4 next = rk4(m, p, ground, steer, rate, accel, grip);
+    if (!m.ok) {
+      Ieee e;
+      next = rk4(e, p, ground, steer, rate, accel, grip);
+    }
+    p = next;
     p.s = clampf_(p.s, -SPEED_MAX, SPEED_MAX);
     steer = clampf_(steer + rate * DT, -STEER_MAX, STEER_MAX);
     ground = probe_surface<LAYERS>(t, p.x, p.y, spot.height, &spot);
     crashed = crashed || spot.clearance < HALF_DIAG || ground.sx * ground.sx + ground.sy * ground.sy > 1.0f;
+    if (sub < SUBSTEPS - 1) touch_rows<LAYERS>(t, spot.cell);
+    if (sub == SUBSTEPS - 2) {  // the last substep ends beside this cell: fetch its waypoint's lines
+      const float* near = t.d + HEADER + (long)(3 * spot.layer + 2) * t.nx * t.ny;
+      touch(near + max((long)spot.cell - t.nx, 0l));
+      touch(near + min((long)spot.cell + t.nx, (long)t.nx * t.ny - 1));
+      touch(t.d + t.route + 4 * nearest(t, spot.layer, spot.cell));
+    }
   }
   if (p.h > PI_F) p.h -= TWO_PI_F;
   if (p.h < -PI_F) p.h += TWO_PI_F;
-  float prog = progress(t, spot.layer, p.x, p.y);
-  float dp = prog - s[(long)PROGRESS * n + i];
+  float prog = progress(t, spot.layer, spot.cell, p.x, p.y);
+  float dp = prog - progress0;
   float half = (float)t.waypoints / 2.0f;
   dp = dp > half ? dp - 2.0f * half : (dp < -half ? dp + 2.0f * half : dp);
   float score = crashed ? -2.0f : ((10.0f * dp) * t.spacing - (0.001f * steer) * steer);
-  float steps = s[(long)STEPS * n + i] + 1.0f;
+  float steps = steps0 + 1.0f;
   float reason = (float)(crashed ? CRASH : (steps >= (float)HORIZON ? TIMEOUT : 0));
   s[(long)X * n + i] = p.x;
   s[(long)Y * n + i] = p.y;
@@ -375,7 +480,7 @@ __device__ __forceinline__ void advance_car(const TrackDev& t, float* s, const f
   s[(long)STEER * n + i] = steer;
   s[(long)STEPS * n + i] = steps;
   s[(long)PROGRESS * n + i] = prog;
-  s[(long)RETURN * n + i] = s[(long)RETURN * n + i] + score;
+  s[(long)RETURN * n + i] = return0 + score;
   reward[i] = score;
   done[i] = reason;
   float heading = p.h, speed = p.s;
@@ -667,8 +772,6 @@ __device__ __forceinline__ float beam_range(const TrackDev& t, const float4* ray
                                             const float2* __restrict__ beam_dir, int max_iters, bool counted,
                                             int car, int beam, int* count_out);
 
-__device__ __forceinline__ float quotient(float a, float b, float y, float q0);
-
 // RN(a / b) for b normal and a zero or normal of either sign, from y = RN(1 / b):
 // the quotient's residual corrections (a sign-symmetric computation), with a
 // zero returned as itself so that -0 / b stays -0.
@@ -735,20 +838,6 @@ __device__ __forceinline__ float beam_range(const TrackDev& t, const float4* ray
     range = march<LAYERS, false, false>(t, ox, oy, oz, dx, dy, dz, descent, inv_descent, max_iters, &count);
   *count_out = count;
   return range;
-}
-
-// RN(a / b) from y = RN(1 / b) and q0 = RN(a * y), by two residual
-// corrections (Markstein, IBM J. Res. Dev. 34(1), 1990): r = a - b q is exact
-// in one fused multiply-add when q is within a few ulps of a / b, and
-// RN(q + r y) is then the correctly rounded quotient once q is faithful,
-// which the first correction makes it. For the march's operands (0 <= a,
-// b >= 0, neither subnormal) this is the IEEE quotient whenever that is
-// finite; for b = 0, an overflowing product or a NaN it gives NaN or +inf.
-// Checked against IEEE division on random and near-midpoint quotients
-// (tests/test_cell_index.py) and by the bit-exact lidar tests.
-__device__ __forceinline__ float quotient(float a, float b, float y, float q0) {
-  const float q1 = __fmaf_rn(__fmaf_rn(-q0, b, a), y, q0);
-  return __fmaf_rn(__fmaf_rn(-q1, b, a), y, q1);
 }
 
 // The march of one beam (racer/sim.mojo:252-266); returns the range.
