@@ -27,6 +27,7 @@ UNITS = {
     "mlp_tc.cu": EXACT,
     "policy.cu": [],
     "policy_tc.cu": [],
+    "update_tc.cu": EXACT,
     "api.cu": [],
     "noalloc.cu": [],
     "tma.cu": [],

@@ -25,6 +25,7 @@
 #include "policy_fwd.h"
 #include "surrogate.h"
 #include "tma.h"
+#include "update_tc.h"
 
 namespace racer_host {
 static thread_local std::string g_error;
@@ -108,6 +109,7 @@ struct racer_trainer {
   void* xb = nullptr;
   int xld = 0;
   CUtensorMap xmaps[MINIBATCHES];
+  UpdateWork fused;  // the fused minibatch's buffers (inputs of at most UPDATE_MAX_IN rows)
   cudaGraphExec_t update_exec = nullptr;
   racer_policy* update_policy = nullptr;
   int update_generation = -1;
@@ -682,6 +684,10 @@ int racer_trainer_create(int n, int beams, int rollout, void* stream, racer_trai
         return rc;
       }
   }
+  if (tr->in_rows <= UPDATE_MAX_IN && (rc = update_work_new(tr->in_rows, tr->batch, &tr->fused))) {
+    racer_trainer_destroy(tr);
+    return rc;
+  }
   if (cudaMallocHost((void**)&tr->c12_host, 2 * EPOCHS * MINIBATCHES * sizeof(float)) != cudaSuccess) {
     set_error("racer_trainer_create: pinned allocation failed");
     tr->c12_host = nullptr;
@@ -713,6 +719,7 @@ int racer_trainer_destroy(racer_trainer* tr) {
     cudaFree(p);
   if (tr->c12_host) cudaFreeHost(tr->c12_host);
   cudaFree(tr->xb);
+  update_work_delete(&tr->fused);
   racer_acts_destroy(tr->acts);
   if (tr->owned && tr->st) cudaStreamDestroy(tr->st);
   delete tr;
@@ -869,6 +876,20 @@ static int update_body(racer_trainer* tr, racer_policy* p) {
   // the minibatches' samples are the same in every epoch: gather them once
   launch_gather_all(tr->in_rows, tr->n, tr->rollout, tr->batch, tr->obs, tr->x, st, tr->xb, tr->xld);
   RACER_LAUNCHED();
+  // BF16 policies of at most UPDATE_MAX_IN inputs: the minibatch in one tile kernel (update_tc.cu), 68 us a
+  // minibatch at 262144 samples x 113 inputs with Adam against 275 in the separate kernels, which wider inputs
+  // keep (a tile's inputs and their weight gradient no longer fit an SM's shared and tensor memory)
+  if (tr->fused.part && policy_is_bf16(p)) {
+    RACER_TRY(launch_update_begin(&tr->fused, tr->n, tr->actions, tr->logp, tr->value, tr->advantage, policy_theta(p), st));
+    for (int k = 0; k < EPOCHS * MINIBATCHES; ++k) {
+      const int m = (k % MINIBATCHES + k / MINIBATCHES) % MINIBATCHES;
+      UpdateDump dump;  // the last minibatch's activations and derivatives stay in the trainer's buffers
+      if (k == EPOCHS * MINIBATCHES - 1) dump = UpdateDump{tr->acts->h1, tr->acts->h2, tr->acts->o, tr->d3};
+      RACER_TRY(launch_update_minibatch(&tr->fused, m, tr->xmaps[m], policy_theta(p), policy_pack(p), tr->grad,
+                                        tr->first, tr->second, tr->c12_dev + 2 * k, tr->stats, dump, policy_err(p), st));
+    }
+    return policy_refresh_on(p, st);
+  }
   for (int epoch = 0; epoch < EPOCHS; ++epoch) {
     for (int m = 0; m < MINIBATCHES; ++m) {
       int rc = minibatch_on(tr, p, (m + epoch) % MINIBATCHES, 1, 0.0f, 1.0f, false);

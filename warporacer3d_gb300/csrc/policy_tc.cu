@@ -99,9 +99,8 @@ __global__ void __launch_bounds__(128, 4)
   uint32_t packed[H / 2];
 #pragma unroll
   for (int k = 0; k < HA; ++k) {
-    const float acc = w2[k] * e0 + w2[HA + k] * e1 + w2[2 * HA + k] * e2;
     const float a = hv[k];
-    const float v = acc * (1.0f - a * a);
+    const float v = tanh_grad(output_grad(w2[k], w2[HA + k], w2[2 * HA + k], e0, e1, e2), a);
     if (live) {
       if (write_f32) d2[(long)k * cols + j] = v;
       h2b[(long)k * ld + j] = __float2bfloat16_rn(a);  // the weight-gradient operand of layer 2
@@ -144,7 +143,7 @@ __global__ void __launch_bounds__(128, 4)
       for (int k = 0; k < 32; ++k) hh[k] = h1[(long)(k0 + k) * cols + j];
 #pragma unroll
       for (int k = 0; k < 32; ++k) {
-        const float g = acc[k0 + k] * (1.0f - hh[k] * hh[k]);
+        const float g = tanh_grad(acc[k0 + k], hh[k]);
         if (write_f32) d1[(long)(k0 + k) * cols + j] = g;
         d1f[(long)(k0 + k) * ld + j] = __float2bfloat16_rn(g);
         h1b[(long)(k0 + k) * ld + j] = __float2bfloat16_rn(hh[k]);  // the weight-gradient operand of layer 1
@@ -185,8 +184,6 @@ int walloc(T** p, size_t count) {
   return 0;
 }
 
-constexpr int MAX_SPLIT_TILES = 296;
-
 }  // namespace
 
 struct BackwardWork {
@@ -208,7 +205,7 @@ int backward_work_new(int in, int cols, BackwardWork** out) {
       (rc = walloc(&w->h2b, (size_t)HA * ld)) || (rc = walloc(&w->d2f, (size_t)H * ld)) ||
       (rc = walloc(&w->d3f, (size_t)16 * ld)) || (rc = walloc(&w->d1f, (size_t)H * ld)) ||
       (rc = walloc(&w->w1ts, (size_t)H * H)) ||
-      (rc = walloc(&w->scratch, (size_t)MAX_SPLIT_TILES * 128 * 64))) {
+      (rc = walloc(&w->scratch, (size_t)WGRAD_SPLITS * 128 * 64))) {
     backward_work_delete(w);
     return rc;
   }
@@ -247,7 +244,7 @@ int wgrad(BackwardWork* w, const CUtensorMap& ta, const CUtensorMap& tb, int mro
           int ldg, int* err, cudaStream_t st) {
   const int kblocks = w->ld / 64 + (w->ld % 64 ? 1 : 0);
   const int tiles = (mrows + 127) / 128;
-  int splits = std::max(1, std::min(kblocks, MAX_SPLIT_TILES / tiles));
+  int splits = std::max(1, std::min(kblocks, WGRAD_SPLITS / tiles));
   const int per = (kblocks + splits - 1) / splits;
   splits = (kblocks + per - 1) / per;
   EpiSplitF32 epi{w->scratch, (long)mrows * nreal, mrows, nreal};

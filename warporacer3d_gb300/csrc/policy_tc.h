@@ -1,9 +1,21 @@
 // BF16 tensor-core backward of the policy MLP (policy_tc.cu).
 #pragma once
+#include "common.cuh"
 #include "tma.h"
 #include <cuda_runtime.h>
 
 namespace racer {
+
+// The batch is split into at most this many ranges of whole 64-sample k-blocks for the weight gradients
+// of up to 128 rows, here and in the fused minibatch (update_tc.cu), whose sums have the same order.
+constexpr int WGRAD_SPLITS = 296;
+
+// The tanh layer's derivative, g (1 - h^2), and the output layer's, W2^T d3 of one unit, in the multiply-adds
+// that both backward kernels (policy_tc.cu, update_tc.cu) use.
+__device__ __forceinline__ float tanh_grad(float g, float h) { return g * __fmaf_rn(-h, h, 1.0f); }
+__device__ __forceinline__ float output_grad(float w0, float w1, float w2, float e0, float e1, float e2) {
+  return __fmaf_rn(w2, e2, __fmaf_rn(w0, e0, w1 * e1));
+}
 
 struct BackwardWork;  // BF16 operand copies, tensor maps and split-K scratch for one batch size
 

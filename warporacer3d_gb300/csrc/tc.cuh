@@ -50,6 +50,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, 
       "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
+// The same box into L2 only; nothing waits for it.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(tmap)),
+               "r"(x), "r"(y)
+               : "memory");
+}
 // 1-D bulk copy of `bytes` (a multiple of 16; both addresses 16-byte aligned)
 // from global into shared memory, completing `bytes` on `bar`.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -127,6 +133,22 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr) {
   d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset: 8 rows x 128 B
   d |= (uint64_t)1 << 46;                    // descriptor version (sm_100 family)
   d |= (uint64_t)2 << 61;                    // swizzle: 128B
+  return d;
+}
+
+// The same 128-byte-swizzled rows read as an MN-major operand: a row holds 64
+// consecutive M (or N) elements of one k, so 8 k's are 1024 bytes, a K step of
+// 16 adds 2048 bytes to the start address, and the next 64 M elements lie
+// mn_stride bytes further on (unused for a 64-wide operand). The instruction
+// descriptor says which operands are MN-major.
+constexpr uint32_t A_MN = 1u << 15, B_MN = 1u << 16;
+__device__ __forceinline__ uint64_t sdesc_mn_sw128(uint32_t saddr, uint32_t mn_stride) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+  d |= (uint64_t)((mn_stride & 0x3FFFFu) >> 4) << 16;  // leading byte offset: 64 M elements
+  d |= (uint64_t)(1024 >> 4) << 32;                    // stride byte offset: 8 k
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
   return d;
 }
 
