@@ -32,7 +32,8 @@ namespace {
 
 
 // Two producer groups of four warps, one k-block in flight each in registers
-// (64 KB of loads an SM, 128 KB with two CTAs), plus one MMA warp. Shared
+// (64 KB of loads an SM, 128 KB with two CTAs), plus one MMA warp; four groups
+// for wide inputs of a few samples, where only a CTA's own latency counts. Shared
 // memory is kept to 54 KB: the SM's L1 is what its resident CTAs leave of 256
 // KB, and the lidar of another rollout chain or stream that shares the SM
 // gathers its cells through it (k_lidar_track at 4096 cars x 1081 beams takes
@@ -41,8 +42,8 @@ namespace {
 // tanh), and no stage is deeper than the loads in flight need. The TMA-staged
 // kernel below (200 KB) in this place made a 64-step rollout of 4096 cars in
 // 16 chains 7.12 ms against 6.45.
+template <int GROUPS>
 struct FwdCfg {
-  static constexpr int GROUPS = 2;
   static constexpr int THREADS = (GROUPS * 4 + 1) * 32;
   static constexpr int MMA_WARP = GROUPS * 4;
   static constexpr int OFF_A = 0;  // GROUPS x A; H = [h | 1 | 0] reuses A[0], A[1]
@@ -61,14 +62,15 @@ struct FwdCfg {
 // four K=16 MMAs of the block and commits to empty[kb % 2]; after the last
 // block it commits to `done`. Warps 0-3 (TMEM lanes 0-127) then run the
 // epilogues and issue layers 2 and 3.
-__global__ void __launch_bounds__(FwdCfg::THREADS, 2)
+template <int GROUPS>
+__global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
     k_mlp_fwd(const float* __restrict__ x, int in, int cols, int c0, int c1,
                                                         const uint4* __restrict__ w0s, int kblocks,
                                                         const uint4* __restrict__ w1s,
                                                         const uint4* __restrict__ w2s, float* h1g, float* h2g,
                                                         float* og, int write_hidden, SampleArgs sa, int* err) {
-  using C = FwdCfg;
-  constexpr int GROUPS = C::GROUPS, THREADS = C::THREADS, MMA_WARP = C::MMA_WARP, OFF_A = C::OFF_A, OFF_B = C::OFF_B,
+  using C = FwdCfg<GROUPS>;
+  constexpr int THREADS = C::THREADS, MMA_WARP = C::MMA_WARP, OFF_A = C::OFF_A, OFF_B = C::OFF_B,
                 OFF_W1 = C::OFF_W1, OFF_W2 = C::OFF_W2, OFF_BAR = C::OFF_BAR;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = tc::smem_u32(smem_raw);
@@ -445,17 +447,18 @@ void launch_pack_weights(const float* theta, int in, uint8_t* pack, cudaStream_t
   k_pack_weights<<<device_sms(), 256, 0, st>>>(theta, in, kb, w0, w1, w2);
 }
 
+template <int GROUPS>
 static cudaError_t fwd_launch(const float* x, int in, int cols, int c0, int c1, int kb, const uint4* w0,
                               const uint4* w1, const uint4* w2, float* h1, float* h2, float* o, int write_hidden,
                               const SampleArgs& sa, int* err, cudaStream_t st) {
-  using C = FwdCfg;
+  using C = FwdCfg<GROUPS>;
   static unsigned long long configured = 0;  // per device
   cudaError_t e = once_per_device(&configured, [] {
-    return cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+    return cudaFuncSetAttribute(k_mlp_fwd<GROUPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
   });
   if (e != cudaSuccess) return e;
   if (c1 <= c0) return cudaSuccess;
-  k_mlp_fwd<<<(c1 - c0 + TILE - 1) / TILE, C::THREADS, C::SMEM_BYTES, st>>>(x, in, cols, c0, c1, w0, kb, w1, w2,
+  k_mlp_fwd<GROUPS><<<(c1 - c0 + TILE - 1) / TILE, C::THREADS, C::SMEM_BYTES, st>>>(x, in, cols, c0, c1, w0, kb, w1, w2,
                                                                                   h1, h2, o, write_hidden, sa, err);
   return cudaGetLastError();
 }
@@ -486,7 +489,12 @@ cudaError_t launch_mlp_fwd(const float* x, int in, int cols, const uint8_t* pack
                                                                    write_hidden, sa, err);
     return cudaGetLastError();
   }
-  return fwd_launch(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
+  // Few tiles in the whole batch (of which [c0, c1) may be one chain's part): four k-blocks in
+  // flight (22 samples x 455 inputs: 14.4 us; two cost 0.8 us more). More tiles share
+  // their SMs with a lidar and leave it the L1.
+  if (kb > 2 && (cols + TILE - 1) / TILE <= 8)
+    return fwd_launch<4>(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
+  return fwd_launch<2>(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
 }
 
 }  // namespace racer
