@@ -80,9 +80,9 @@ void launch_rowsum(const float* x, int rows, int cols, long ld, float* out, floa
                    cudaStream_t st);
 void launch_moments(const float* adv, long count, float* stats, float* scratch, cudaStream_t st);
 
-// mlp.cu (policy GEMMs)
-void launch_sgemm(const float* A, int lda, const float* B, int ldb, float* C, int ldc, int M, int N, int K,
-                  int squash, cudaStream_t st);
+// mlp.cu (the policy in FP32): x [in, cols] -> h1, h2 [65, cols] (row 64, the bias input, is read), o [3, cols]
+void launch_fwd_f32(int in, const float* theta, const float* x, int cols, float* h1, float* h2, float* o,
+                    cudaStream_t st);
 void launch_backward(int in, const float* theta, const float* x, int cols, const float* h1, const float* h2,
                      const float* d3, float* d2, float* d1, float* grad, float* scratch, cudaStream_t st);
 // The FP32 weight-gradient GEMMs split K over the batch into at most SPLIT_CTAS / tiles ranges of

@@ -98,10 +98,7 @@ int policy_forward(racer_policy* p, const float* x, int cols, float* h1, float* 
       racer_host::set_error("policy forward: column ranges need the BF16 path");
       return 1;
     }
-    const int in = p->in, w1 = H * in, w2 = w1 + H * HA;
-    launch_sgemm(p->theta, in, x, cols, h1, cols, H, cols, in, 1, st);
-    launch_sgemm(p->theta + w1, HA, h1, cols, h2, cols, H, cols, HA, 1, st);
-    launch_sgemm(p->theta + w2, HA, h2, cols, o, cols, OUT, cols, HA, 0, st);
+    launch_fwd_f32(p->in, p->theta, x, cols, h1, h2, o, st);
     if (sa && sa->actions)
       launch_sample(cols, sa->seed, o, sa->log_std, sa->actions, sa->logp, sa->value, sa->deterministic,
                     sa->step_base, sa->step_add, st);
