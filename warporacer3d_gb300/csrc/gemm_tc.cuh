@@ -1,13 +1,18 @@
 // Generic tcgen05 GEMM: D[M, N] = A[M, K] . B[N, K]^T with BF16 operands
-// (both K-major, loaded by TMA as 128B-swizzled 64-wide k-blocks) and FP32
-// accumulation in TMEM, followed by a caller-supplied epilogue.
+// (loaded by TMA as 128B-swizzled 64-wide k-blocks) and FP32 accumulation in
+// TMEM, followed by a caller-supplied epilogue. Both operands lie K-contiguous
+// in memory, or (MN) K-strided: A as [K, M] rows, B as [K, N] rows, the layout
+// of sample-major activations in a weight gradient, whose K is the batch. The
+// products and their order are the same either way.
 //
 // Persistent: one CTA per SM walks the 128 x BN output tiles (and split-K
 // ranges) blockIdx.x, blockIdx.x + gridDim.x, ... Warp 0 is the TMA producer
 // (a ring of stages across tiles), warp 1 allocates two TMEM accumulators and
-// issues the MMAs (one thread), warps 2-9 are the epilogue: two warps per
-// 32-lane TMEM quadrant, each taking half of the columns. The accumulator of
-// tile i + 1 fills while the epilogue drains tile i. Every mbarrier wait is
+// issues the MMAs (one thread), the other warps are the epilogue: two or four
+// per 32-lane TMEM quadrant, each taking its share of the columns (an epilogue
+// is latency-bound: the learned lidar's loss at 8192 x 1472 takes 44 us with 16
+// warps and 55 with eight). The accumulator of tile i + 1 fills while the
+// epilogue drains tile i. Every mbarrier wait is
 // bounded and a timeout sets *err.
 #pragma once
 #include <cuda.h>
@@ -31,17 +36,26 @@ struct GemmCfg {
   static constexpr int ACC_COLS = BN < 16 ? 16 : BN;
   static constexpr int TMEM_COLS = 2 * ACC_COLS < 32 ? 32 : 2 * ACC_COLS;
   static constexpr int SMEM = STAGES * STAGE_BYTES + 256 + 1024;
-  static constexpr int EPI_WARPS = 8;
+  static constexpr int EPI_WARPS = BN >= 256 ? 16 : 8;  // per 32-lane quadrant: four or two, each a share of the columns
   static constexpr int THREADS = (2 + EPI_WARPS) * 32;
 };
 
 // Epilogue contract: operator()(m, n, v, z) with v[0..15] = D[m][n .. n+15] of split z, called
 // by all 32 lanes of an epilogue warp together (lane = row); callers mask
-// m >= M and n + j >= N themselves.
-template <int BN, typename Epi>
+// m >= M and n + j >= N themselves. Each thread has its own copy, which may
+// hold state; finish(), where there is one, is called by whole warps once
+// their tiles are done.
+template <typename Epi>
+__device__ __forceinline__ auto epi_finish(Epi& e, int) -> decltype(e.finish()) {
+  e.finish();
+}
+template <typename Epi>
+__device__ __forceinline__ void epi_finish(Epi&, long) {}
+
+template <int BN, typename Epi, bool MN>
 __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
     k_gemm(const __grid_constant__ CUtensorMap ta, const __grid_constant__ CUtensorMap tb, int mtiles, int ntiles,
-           int splits, int kblocks, int kb_per_split, Epi epi, int* err) {
+           int splits, int kblocks, int kb_per_split, Epi epi_arg, int* err) {
   using C = GemmCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = tc::smem_u32(smem_raw);
@@ -86,12 +100,20 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
         if (it >= (uint32_t)C::STAGES && !tc::mbar_wait(&empty[s], ((it / C::STAGES) - 1) & 1)) ok = false;
         uint8_t* st = smem + s * C::STAGE_BYTES;
         tc::mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
-        tc::tma_load_2d(st, &ta, kb * 64, mt * C::BM, &full[s]);
-        tc::tma_load_2d(st + C::A_BYTES, &tb, kb * 64, nt * BN, &full[s]);
+        if (MN) {  // 64 k's by 64 elements of M or N a box
+#pragma unroll
+          for (int i = 0; i < C::BM / 64; ++i) tc::tma_load_2d(st + i * 8192, &ta, mt * C::BM + 64 * i, kb * 64, &full[s]);
+#pragma unroll
+          for (int i = 0; i < BN / 64; ++i)
+            tc::tma_load_2d(st + C::A_BYTES + i * 8192, &tb, nt * BN + 64 * i, kb * 64, &full[s]);
+        } else {
+          tc::tma_load_2d(st, &ta, kb * 64, mt * C::BM, &full[s]);
+          tc::tma_load_2d(st + C::A_BYTES, &tb, kb * 64, nt * BN, &full[s]);
+        }
       }
     }
   } else if (warp == 1 && lane == 0) {
-    const uint32_t idesc = tc::idesc_bf16(C::BM, BN);
+    const uint32_t idesc = tc::idesc_bf16(C::BM, BN) | (MN ? tc::A_MN | tc::B_MN : 0u);
     uint32_t it = 0, local = 0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
       const int z = tile / (ntiles * mtiles);
@@ -107,7 +129,8 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
         const uint32_t a = tc::smem_u32(smem + s * C::STAGE_BYTES), b = a + C::A_BYTES;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          tc::mma_bf16(d, tc::sdesc_sw128(a + 32 * k), tc::sdesc_sw128(b + 32 * k), idesc,
+          tc::mma_bf16(d, MN ? tc::sdesc_mn_sw128(a + 2048 * k, 8192) : tc::sdesc_sw128(a + 32 * k),
+                       MN ? tc::sdesc_mn_sw128(b + 2048 * k, 8192) : tc::sdesc_sw128(b + 32 * k), idesc,
                        (kb > kb0 || k > 0) ? 1u : 0u);
         tc::mma_commit(&empty[s]);
       }
@@ -115,9 +138,10 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
     }
   } else if (warp >= 2) {
     const int q = warp & 3;                // TMEM lane quadrant
-    const int half = (warp - 2) >> 2;      // which half of the columns
-    constexpr int HALF = C::ACC_COLS / 2;  // >= 8
+    const int half = (warp - 2) >> 2;      // which share of the columns
+    constexpr int HALF = C::ACC_COLS / (C::EPI_WARPS / 4);  // >= 8
     uint32_t local = 0;
+    Epi epi = epi_arg;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
       const int nt = tile % ntiles, mt = (tile / ntiles) % mtiles, z = tile / (ntiles * mtiles);
       const int kb0 = z * kb_per_split, kb1 = min(kblocks, kb0 + kb_per_split);
@@ -153,6 +177,8 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
       tc::tc_fence_before();
       tc::mbar_arrive(&aempty[buf]);
     }
+    __syncwarp();
+    epi_finish(epi, 0);
   }
   tc::tc_fence_before();
   __syncthreads();
@@ -161,20 +187,21 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
 }
 
 // Sets the kernel's shared-memory limit once per device (call before capturing a launch into a graph).
-template <int BN, typename Epi>
+template <int BN, typename Epi, bool MN = false>
 cudaError_t gemm_configure() {
   static unsigned long long configured = 0;
   return once_per_device(&configured, [] {
-    return cudaFuncSetAttribute(k_gemm<BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM);
+    return cudaFuncSetAttribute(k_gemm<BN, Epi, MN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM);
   });
 }
 
-// Launch over an M x N output with K = kblocks * 64 split into `splits` ranges.
-template <int BN, typename Epi>
+// Launch over an M x N output with K = kblocks * 64 split into `splits` ranges. The tensor maps'
+// boxes: K-contiguous operands 64 x 128 (A) and 64 x BN (B); MN ones 64 x 64.
+template <int BN, typename Epi, bool MN = false>
 cudaError_t gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int kblocks, int splits,
                         const Epi& epi, int* err, cudaStream_t st) {
   using C = GemmCfg<BN>;
-  cudaError_t ce = gemm_configure<BN, Epi>();
+  cudaError_t ce = gemm_configure<BN, Epi, MN>();
   if (ce != cudaSuccess) return ce;
   const int sms = device_sms();
   if (splits < 1) splits = 1;
@@ -182,8 +209,8 @@ cudaError_t gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int
   splits = (kblocks + per - 1) / per;
   const int mtiles = (M + C::BM - 1) / C::BM, ntiles = (N + BN - 1) / BN;
   const int tiles = mtiles * ntiles * splits;
-  k_gemm<BN, Epi><<<tiles < sms ? tiles : sms, C::THREADS, C::SMEM, st>>>(ta, tb, mtiles, ntiles, splits, kblocks,
-                                                                          per, epi, err);
+  k_gemm<BN, Epi, MN><<<tiles < sms ? tiles : sms, C::THREADS, C::SMEM, st>>>(ta, tb, mtiles, ntiles, splits, kblocks,
+                                                                              per, epi, err);
   return cudaGetLastError();
 }
 

@@ -37,11 +37,14 @@
 // Inference writes the clamped world profile as FP16 rows per car and a
 // gather kernel turns them into the beam rows of obs.
 //
-// Activations are sample-major BF16 for the forward GEMMs and also written
-// feature-major (batch contiguous) for the weight-gradient GEMMs; every GEMM
-// is the generic tcgen05 kernel (BF16 operands by TMA, FP32 accumulation in
-// TMEM) with an epilogue that applies tanh/bias, the loss gradient, the tanh
-// derivative or the split-K partial store. Master weights and Adam are FP32.
+// Activations and their gradients are sample-major BF16: K-contiguous operands
+// of the forward and data-gradient GEMMs and, read MN-major, the operands of
+// the weight-gradient GEMMs, whose K is the batch. (A feature-major copy of
+// each for the latter cost the epilogues a 2-byte store per value: 50 us for
+// an 8192 x 512 gradient against 15 us without.) Every GEMM is the generic
+// tcgen05 kernel (BF16 operands by TMA, FP32 accumulation in TMEM) with an
+// epilogue that applies tanh/bias, the loss gradient, the tanh derivative or
+// the split-K partial store. Master weights and Adam are FP32.
 //
 // Training poses are uniform over the drivable cells (clearance > 0) of every
 // layer with uniform heading; their labels come from the exact tracer
@@ -111,134 +114,173 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// H = tanh(v + bias) -> sample-major hs [M, lds] and feature-major hf [N, ldf] (either may be null).
-struct EpiTanhOut {
-  bf16* hs;
-  int lds;
-  bf16* hf;
-  int ldf;
-  const float* bias;
-  int M, N;
-  __device__ void operator()(int m, int n, const float* v, int z) const {
-    if (m >= M) return;
-    float h[16];
+// The sums over a warp's 32 lanes of 16 values each, column j = 8 (lane >> 4) + 4 (lane >> 3 & 1) + 2 (lane >> 2 & 1)
+// + (lane >> 1 & 1) in the lane (twice): halving exchanges, 16 shuffles where a sum per column takes 80.
+__device__ __forceinline__ float column_sums(const float* v) {
+  const int lane = threadIdx.x & 31;
+  float a[8], b[4], c[2], d;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) h[j] = (n + j < N) ? tc::tanh_fast(v[j] + (bias ? bias[n + j] : 0.0f)) : 0.0f;
-    if (hs && n < N) {  // N is a multiple of 16: a chunk is wholly inside or outside
-      uint4 a = make_uint4(tc::pack_bf16(h[0], h[1]), tc::pack_bf16(h[2], h[3]), tc::pack_bf16(h[4], h[5]),
-                           tc::pack_bf16(h[6], h[7]));
-      uint4 b = make_uint4(tc::pack_bf16(h[8], h[9]), tc::pack_bf16(h[10], h[11]), tc::pack_bf16(h[12], h[13]),
-                           tc::pack_bf16(h[14], h[15]));
-      uint4* dst = reinterpret_cast<uint4*>(hs + (long)m * lds + n);
-      dst[0] = a;
-      dst[1] = b;
+  for (int j = 0; j < 8; ++j)
+    a[j] = (lane & 16 ? v[j + 8] : v[j]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? v[j] : v[j + 8], 16);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    b[j] = (lane & 8 ? a[j + 4] : a[j]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? a[j] : a[j + 4], 8);
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    c[j] = (lane & 4 ? b[j + 2] : b[j]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? b[j] : b[j + 2], 4);
+  d = (lane & 2 ? c[1] : c[0]) + __shfl_xor_sync(0xffffffffu, lane & 2 ? c[0] : c[1], 2);
+  return d + __shfl_xor_sync(0xffffffffu, d, 1);
+}
+// out[n + j] += the warp's sum of column j, for n + j < N.
+__device__ __forceinline__ void add_columns(const float* v, float* out, int n, int N) {
+  const float s = column_sums(v);
+  const int lane = threadIdx.x & 31;
+  const int j = 8 * (lane >> 4) + 4 * ((lane >> 3) & 1) + 2 * ((lane >> 2) & 1) + ((lane >> 1) & 1);
+  if (!(lane & 1) && n + j < N) atomicAdd(out + n + j, s);
+}
+
+__device__ __forceinline__ void store16(bf16* dst, const float* g) {
+  uint4* d = reinterpret_cast<uint4*>(dst);
+  d[0] = make_uint4(tc::pack_bf16(g[0], g[1]), tc::pack_bf16(g[2], g[3]), tc::pack_bf16(g[4], g[5]),
+                    tc::pack_bf16(g[6], g[7]));
+  d[1] = make_uint4(tc::pack_bf16(g[8], g[9]), tc::pack_bf16(g[10], g[11]), tc::pack_bf16(g[12], g[13]),
+                    tc::pack_bf16(g[14], g[15]));
+}
+
+// out[j] = bias[n + j], 0 past N; bias + n is 16-byte aligned.
+__device__ __forceinline__ void load_bias(const float* bias, int n, int N, float* out) {
+  if (n + 16 <= N) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 f = __ldg(reinterpret_cast<const float4*>(bias + n) + q);
+      out[4 * q] = f.x, out[4 * q + 1] = f.y, out[4 * q + 2] = f.z, out[4 * q + 3] = f.w;
     }
-    if (hf) {
+  } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (n + j < N) hf[(long)(n + j) * ldf + m] = __float2bfloat16_rn(h[j]);
+    for (int j = 0; j < 16; ++j) out[j] = n + j < N ? __ldg(bias + n + j) : 0.0f;
+  }
+}
+
+// A thread's loss sums over its tiles: FP32 within 16 columns, beyond that FP32 with the rounding errors carried
+// (Knuth's two-sum; FP64 additions are slow here), added to sums[0], sums[1] once per warp in FP64.
+struct LossSums {
+  float s[2] = {0.0f, 0.0f}, c[2] = {0.0f, 0.0f};
+  double* sums;
+  __device__ __forceinline__ void add(float se, float ae) {
+    const float x[2] = {se, ae};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float t = s[k] + x[k], b = t - s[k];
+      c[k] += (s[k] - (t - b)) + (x[k] - b);
+      s[k] = t;
+    }
+  }
+  __device__ __forceinline__ void flush() {
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      double d = (double)s[k] + (double)c[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      if ((threadIdx.x & 31) == 0) atomicAdd(sums + k, d);
     }
   }
 };
 
-// Output layer in training: y = v + b4, e = y - target, g = scale * e (MSE gradient).
-// Writes g sample-major [M, ldgs] and feature-major [npad rows, ldgf] (zero past N),
-// accumulates the bias gradient and the sums of e^2 and |e|.
+// H = tanh(v + bias) -> hs [M, lds].
+struct EpiTanhOut {
+  bf16* hs;
+  int lds;
+  const float* bias;
+  int M, N;
+  __device__ void operator()(int m, int n, const float* v, int z) const {
+    if (m >= M) return;
+    if (n >= N) return;  // N is a multiple of 16: a chunk is wholly inside or outside
+    float h[16], b[16];
+    if (bias) load_bias(bias, n, N, b);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) h[j] = tc::tanh_fast(v[j] + (bias ? b[j] : 0.0f));
+    store16(hs + (long)m * lds + n, h);
+  }
+};
+
+// Output layer in training: y = v + b4, e = y - target, g = scale * e (MSE gradient; with huber > 0 e clamped to
+// +-huber). Writes g [M, ldgs] (zero past N), accumulates the bias gradient and the sums of e^2 and |e|. The target of
+// (row m, column n + j) is target[(n + j) * ldt + m] (car frame) or, where window says the column is one that the
+// row's beams read, rows[m * ldgs + n + j] (world frame; other columns' gradient is 0).
+template <bool WORLD>
 struct EpiLoss {
-  const float* target;  // [N, ldt] feature-major
+  const float* target;  // car frame: [N, ldt]; world frame: [M, ldgs], every row's targets at its own world samples
   int ldt;
+  const int* k0;  // world frame: the row's first world sample; its beams read k0 .. k0 + beams - 1 modulo N
+  int beams;
   const float* bias;
   int M, N;
   float scale;
   bf16* gs;
-  int ldgs;
-  bf16* gf;
-  int ldgf;
+  int ldgs;  // also the columns stored (a multiple of 16; past N they are zero)
   float* dbias;
-  double* sums;
-  int npad;     // columns stored (a multiple of 16; past N they are zero)
-  float huber;  // > 0: Huber loss with this threshold (range units), its gradient e clamped to +-huber
-  __device__ void operator()(int m, int n, const float* v, int z) const {
+  float huber;
+  LossSums total;
+  __device__ __forceinline__ void operator()(int m, int n, const float* v, int z) {
     const bool row = m < M;
-    float g[16], se = 0.0f, ae = 0.0f;
+    float g[16], t[16], bb[16], se = 0.0f, ae = 0.0f;
+    int first = 0;
+    if (WORLD) {
+      if (n >= ldgs) return;  // n is a multiple of 16, ldgs of 64
+      first = row ? __ldg(k0 + m) : 0;
+      const float4* src = reinterpret_cast<const float4*>(target + (long)m * ldgs + n);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 f = row ? __ldg(src + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        t[4 * q] = f.x, t[4 * q + 1] = f.y, t[4 * q + 2] = f.z, t[4 * q + 3] = f.w;
+      }
+    }
+    load_bias(bias, n, N, bb);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       g[j] = 0.0f;
-      if (row && n + j < N) {
-        float e = (v[j] + bias[n + j]) - target[(long)(n + j) * ldt + m];
+      int b = n + j - first;
+      if (WORLD && b < 0) b += N;
+      if (row && n + j < N && (!WORLD || b < beams)) {
+        const float e = (v[j] + bb[j]) - (WORLD ? t[j] : target[(long)(n + j) * ldt + m]);
         se += e * e;
         ae += fabsf(e);
         g[j] = scale * (huber > 0.0f ? fminf(fmaxf(e, -huber), huber) : e);
       }
     }
-    if (row && n < npad) {
-      uint4 a = make_uint4(tc::pack_bf16(g[0], g[1]), tc::pack_bf16(g[2], g[3]), tc::pack_bf16(g[4], g[5]),
-                           tc::pack_bf16(g[6], g[7]));
-      uint4 b = make_uint4(tc::pack_bf16(g[8], g[9]), tc::pack_bf16(g[10], g[11]), tc::pack_bf16(g[12], g[13]),
-                           tc::pack_bf16(g[14], g[15]));
-      uint4* dst = reinterpret_cast<uint4*>(gs + (long)m * ldgs + n);
-      dst[0] = a;
-      dst[1] = b;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) gf[(long)(n + j) * ldgf + m] = __float2bfloat16_rn(g[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      float s = warp_sum(g[j]);
-      if ((threadIdx.x & 31) == 0 && n + j < N) atomicAdd(dbias + n + j, s);
-    }
-    se = warp_sum(se);
-    ae = warp_sum(ae);
-    if ((threadIdx.x & 31) == 0) {
-      atomicAdd(sums, (double)se);
-      atomicAdd(sums + 1, (double)ae);
-    }
+    if (row && n < ldgs) store16(gs + (long)m * ldgs + n, g);
+    add_columns(g, dbias, n, N);
+    total.add(se, ae);
   }
+  __device__ __forceinline__ void finish() { total.flush(); }
 };
 
-// Back through tanh: g = v * (1 - h^2) with h from hs [M, ldh]; writes gs (optional) and gf,
-// accumulates the bias gradient (optional).
+// Back through tanh: g = v * (1 - h^2) with h from hs [M, ldh]; writes gs [M, ldgs], accumulates the bias gradient
+// (optional).
 struct EpiDTanh {
   const bf16* hs;
   int ldh;
   bf16* gs;
   int ldgs;
-  bf16* gf;
-  int ldgf;
   float* dbias;
   int M, N;
-  __device__ void operator()(int m, int n, const float* v, int z) const {
+  __device__ __forceinline__ void operator()(int m, int n, const float* v, int z) const {
+    if (n >= N) return;  // N is a multiple of 16
     const bool row = m < M;
     float g[16];
+    uint32_t h[8] = {};
+    if (row) {
+      const uint4* src = reinterpret_cast<const uint4*>(hs + (long)m * ldh + n);
+      *reinterpret_cast<uint4*>(h) = src[0];
+      *reinterpret_cast<uint4*>(h + 4) = src[1];
+    }
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
-      g[j] = 0.0f;
-      if (row && n + j < N) {
-        float h = __bfloat162float(hs[(long)m * ldh + n + j]);
-        g[j] = v[j] * (1.0f - h * h);
-      }
+      const float t = __uint_as_float(j & 1 ? h[j >> 1] & 0xffff0000u : h[j >> 1] << 16);
+      g[j] = row ? v[j] * (1.0f - t * t) : 0.0f;
     }
-    if (row && n < N) {
-      if (gs) {
-        uint4 a = make_uint4(tc::pack_bf16(g[0], g[1]), tc::pack_bf16(g[2], g[3]), tc::pack_bf16(g[4], g[5]),
-                             tc::pack_bf16(g[6], g[7]));
-        uint4 b = make_uint4(tc::pack_bf16(g[8], g[9]), tc::pack_bf16(g[10], g[11]), tc::pack_bf16(g[12], g[13]),
-                             tc::pack_bf16(g[14], g[15]));
-        uint4* dst = reinterpret_cast<uint4*>(gs + (long)m * ldgs + n);
-        dst[0] = a;
-        dst[1] = b;
-      }
-#pragma unroll
-      for (int j = 0; j < 16; ++j)
-        if (n + j < N) gf[(long)(n + j) * ldgf + m] = __float2bfloat16_rn(g[j]);
-    }
-    if (dbias) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        float s = warp_sum(g[j]);
-        if ((threadIdx.x & 31) == 0 && n + j < N) atomicAdd(dbias + n + j, s);
-      }
-    }
+    if (row) store16(gs + (long)m * ldgs + n, g);
+    if (dbias) add_columns(g, dbias, n, N);
   }
 };
 
@@ -265,28 +307,6 @@ struct EpiInfer {
   }
 };
 
-// World frame, training: y[m * ldy + n] = v + b4 for n < N (unclamped, FP32), 0 past N.
-struct EpiWorldTrain {
-  float* y;
-  int ldy;
-  const float* bias;
-  int M, N;
-  __device__ void operator()(int m, int n, const float* v, int z) const {
-    if (m >= M || n >= ldy) return;  // n is a multiple of 16, ldy of 64
-    float4* dst = reinterpret_cast<float4*>(y + (long)m * ldy + n);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float t[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int o = n + 4 * q + j;
-        t[j] = o < N ? v[4 * q + j] + bias[o] : 0.0f;
-      }
-      dst[q] = make_float4(t[0], t[1], t[2], t[3]);
-    }
-  }
-};
-
 // World frame, layered inference: the world profile of row m into out [M, ldo]
 // (FP16) and the row's smallest range in its field of view into minr.
 struct EpiWorldInfer {
@@ -310,7 +330,7 @@ struct EpiWorldInfer {
   }
 };
 
-// ray frames [2, count] -> encoded inputs, sample-major x [count, 64] and feature-major xf [64, count]:
+// ray frames [2, count] -> encoded inputs x [count, 64]:
 //   0..7    x', y', z, sin h, cos h, [layer 0], [layer 1], 1
 //   8..47   sin/cos(2^k pi x'), sin/cos(2^k pi y') for k = 0..9  (Fourier features,
 //           Tancik et al. 2020: a plain MLP on raw coordinates fits the
@@ -342,20 +362,18 @@ __device__ __forceinline__ void encode(float xn, float yn, float z, float sh, fl
   f[60] = f[61] = f[62] = f[63] = 0.0f;
 }
 
-__global__ void k_features(const float4* __restrict__ ray, int count, Norm nm, bf16* x, bf16* xf) {
+__device__ __forceinline__ void store_inputs(const float* f, int i, bf16* x) {
+#pragma unroll
+  for (int q = 0; q < NIN / 16; ++q) store16(x + (long)i * NIN + 16 * q, f + 16 * q);
+}
+
+__global__ void k_features(const float4* __restrict__ ray, int count, Norm nm, bf16* x) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 r0 = ray[i], r1 = ray[count + i];
   float f[NIN];
   encode((r0.x - nm.xc) * nm.inv_xs, (r0.y - nm.yc) * nm.inv_ys, r0.z, r1.x, r0.w, r1.w, f);
-  uint4* row = reinterpret_cast<uint4*>(x + (long)i * NIN);
-#pragma unroll
-  for (int q = 0; q < NIN / 8; ++q)
-    row[q] = make_uint4(tc::pack_bf16(f[8 * q], f[8 * q + 1]), tc::pack_bf16(f[8 * q + 2], f[8 * q + 3]),
-                        tc::pack_bf16(f[8 * q + 4], f[8 * q + 5]), tc::pack_bf16(f[8 * q + 6], f[8 * q + 7]));
-  if (xf)
-#pragma unroll
-    for (int k = 0; k < NIN; ++k) xf[(long)k * count + i] = __float2bfloat16_rn(f[k]);
+  store_inputs(f, i, x);
 }
 
 // The feature grids of `layer` at (ox, oy), level by level, into f[0 .. 39].
@@ -382,24 +400,13 @@ __device__ __forceinline__ void grid_features(const GridGeom& gg, const float* _
   }
 }
 
-__device__ __forceinline__ void store_inputs(const float* f, int i, int count, bf16* x, bf16* xf) {
-  uint4* row = reinterpret_cast<uint4*>(x + (long)i * NIN);
-#pragma unroll
-  for (int q = 0; q < NIN / 8; ++q)
-    row[q] = make_uint4(tc::pack_bf16(f[8 * q], f[8 * q + 1]), tc::pack_bf16(f[8 * q + 2], f[8 * q + 3]),
-                        tc::pack_bf16(f[8 * q + 4], f[8 * q + 5]), tc::pack_bf16(f[8 * q + 6], f[8 * q + 7]));
-  if (xf)
-#pragma unroll
-    for (int k = 0; k < NIN; ++k) xf[(long)k * count + i] = __float2bfloat16_rn(f[k]);
-}
-
 // Car frame with feature grids (frame 2): ray frames [2, count] -> encoded inputs:
 //   0..39   the feature grids of the origin's layer at (x, y), level by level
 //   40..47  x', y', z, sin h, cos h, [layer 0], [layer 1], 1
 //   48..55  sin/cos(j h) for j = 2..5
 //   56..63  sin/cos(2^k pi x'), sin/cos(2^k pi y') for k = 0, 1
 __global__ void k_features_cargrid(const float4* __restrict__ ray, int count, Norm nm, GridGeom gg,
-                                   const float* __restrict__ grid, bf16* x, bf16* xf) {
+                                   const float* __restrict__ grid, bf16* x) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 r0 = ray[i], r1 = ray[count + i];
@@ -422,7 +429,7 @@ __global__ void k_features_cargrid(const float4* __restrict__ ray, int count, No
   sincospif(yn, &f[58], &f[59]);
   sincospif(2.0f * xn, &f[60], &f[61]);
   sincospif(2.0f * yn, &f[62], &f[63]);
-  store_inputs(f, i, count, x, xf);
+  store_inputs(f, i, x);
 }
 
 // World frame: ray frames [2, count] -> encoded inputs (see the top of this file):
@@ -431,7 +438,7 @@ __global__ void k_features_cargrid(const float4* __restrict__ ray, int count, No
 //   46..61  sin/cos(2^k pi x'), sin/cos(2^k pi y') for k = 0..3
 //   62, 63  sin/cos(2 pi phase)
 __global__ void k_features_world(const float4* __restrict__ ray, int count, Norm nm, GridGeom gg,
-                                 const float* __restrict__ grid, int K, bf16* x, bf16* xf) {
+                                 const float* __restrict__ grid, int K, bf16* x) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 r0 = ray[i], r1 = ray[count + i];
@@ -455,62 +462,34 @@ __global__ void k_features_world(const float4* __restrict__ ray, int count, Norm
   float phase;
   world_phase(r1.x, r0.w, K, &phase);
   sincospif(2.0f * phase, &f[62], &f[63]);
-  store_inputs(f, i, count, x, xf);
+  store_inputs(f, i, x);
 }
 
-// World frame, training loss: one thread per sample m and 64 world samples
-// (blockIdx.y: columns 64 y .. 64 y + 63). Beam b's prediction is
-// y[m][(k0 + b) mod K] (y from EpiWorldTrain, ldy = npad); the loss gradient
-// (scale times the error, clamped to +-huber when huber > 0) goes to that
-// world sample, and every world sample no beam reads gets 0. Writes the
-// gradient sample-major gs [B, npad] and feature-major gf [npad, B] (BF16),
-// sums the output bias gradient and the sums of e^2 and |e| (range units).
-__global__ void __launch_bounds__(128) k_world_loss(const float* __restrict__ y, const float* __restrict__ target,
-                                                    const float4* __restrict__ ray, int B, int beams, int K, int npad,
-                                                    float scale, float huber, bf16* gs, bf16* gf, float* dbias,
-                                                    double* sums) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool row = m < B;
-  int k0 = 0;
-  if (row) {
+// World frame, training: every sample's labels at the world samples its beams read, rows[m * ld + (k0 + b) mod K] =
+// target[b * B + m], and k0. A block turns 32 samples x 32 beams over in shared memory: 128-byte rows in, runs of 32
+// world samples out (the loss epilogue reads whole rows; reading the labels from there took a 32-byte sector a value).
+__global__ void __launch_bounds__(256) k_world_targets(const float* __restrict__ target, const float4* __restrict__ ray,
+                                                       int B, int beams, int K, int ld, float* rows, int* k0) {
+  __shared__ float tile[32][33];
+  __shared__ int first[32];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, m0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
+  if (row == 0) {
     float ph;
-    k0 = world_phase(ray[B + m].x, ray[m].w, K, &ph);
+    const int m = m0 + lane;
+    first[lane] = m < B ? world_phase(ray[B + m].x, ray[m].w, K, &ph) : 0;
+    if (blockIdx.y == 0 && m < B) k0[m] = first[lane];
   }
-  float se = 0.0f, ae = 0.0f;
-  const int c0 = 64 * blockIdx.y;
-  for (int w0 = c0; w0 < c0 + 64 && w0 < npad; w0 += 8) {
-    float g[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int w = w0 + j;
-      g[j] = 0.0f;
-      int b = w - k0;
-      if (b < 0) b += K;
-      if (row && w < K && b < beams) {
-        const float e = y[(long)m * npad + w] - target[(long)b * B + m];
-        se += e * e;
-        ae += fabsf(e);
-        g[j] = scale * (huber > 0.0f ? fminf(fmaxf(e, -huber), huber) : e);
-      }
-    }
-    if (row) {
-      *reinterpret_cast<uint4*>(gs + (long)m * npad + w0) =
-          make_uint4(tc::pack_bf16(g[0], g[1]), tc::pack_bf16(g[2], g[3]), tc::pack_bf16(g[4], g[5]),
-                     tc::pack_bf16(g[6], g[7]));
+  for (int r = row; r < 32; r += 8)
+    tile[r][lane] = b0 + r < beams && m0 + lane < B ? __ldcs(target + (long)(b0 + r) * B + m0 + lane) : 0.0f;
+  __syncthreads();
 #pragma unroll
-      for (int j = 0; j < 8; ++j) gf[(long)(w0 + j) * B + m] = __float2bfloat16_rn(g[j]);
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float t = warp_sum(g[j]);
-      if ((threadIdx.x & 31) == 0 && w0 + j < K) atomicAdd(dbias + w0 + j, t);
-    }
-  }
-  se = warp_sum(se);
-  ae = warp_sum(ae);
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(sums, (double)se);
-    atomicAdd(sums + 1, (double)ae);
+  for (int r = row; r < 32; r += 8) {
+    const int m = m0 + r, b = b0 + lane;
+    if (m >= B || b >= beams) continue;
+    int w = first[r] + b;
+    if (w >= K) w -= K;
+    rows[(long)m * ld + w] = tile[lane][r];
   }
 }
 
@@ -627,13 +606,17 @@ __global__ void k_sample_poses(const int2* cells, int ncells, int count, uint64_
   poses[i] = make_float4(x, y, h, (float)c.y);
 }
 
-// Sum of split-K partials into a row-major [Mreal, N] gradient block.
-__global__ void k_reduce_splits(const float* P, int splits, long mn, int N, int Mreal, float* out) {
-  long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long)Mreal * N) return;
-  float acc = 0.0f;
-  for (int z = 0; z < splits; ++z) acc += P[(long)z * mn + e];
-  out[e] = acc;
+// Sum of split-K partials into a row-major gradient block of `count` floats (a multiple of 4), four per thread.
+__global__ void k_reduce_splits(const float* __restrict__ P, int splits, long mn, long count, float* out) {
+  const long e = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
+  if (e >= count) return;
+  float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 8
+  for (int z = 0; z < splits; ++z) {
+    const float4 v = __ldcs(reinterpret_cast<const float4*>(P + (long)z * mn + e));
+    acc.x += v.x, acc.y += v.y, acc.z += v.z, acc.w += v.w;
+  }
+  *reinterpret_cast<float4*>(out + e) = acc;  // every block of the parameters starts at a multiple of 4
 }
 
 // Parameter block: W1 [H, 64] | W2 [H, H] | b2 | W3 [H, H] | b3 | W4 [nout, H] |
@@ -678,6 +661,18 @@ __global__ void k_refresh(const float* __restrict__ th, Layout L, bf16* w1b, bf1
       w4t[(long)i * L.npad + o] = v;
     }
   }
+}
+
+// What a gradient adds up in place, at zero: the biases' gradients (b4 and the feature grids lie at the end) and the
+// loss sums.
+__global__ void k_zero_sums(float* grad, Layout L, double* sums) {
+  const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long)gridDim.x * blockDim.x;
+  for (long i = i0; i < L.H; i += stride) grad[L.b2 + i] = grad[L.b3 + i] = 0.0f;
+  const long quads = (L.total - L.b4) / 4;  // b4 is a multiple of 4
+  for (long i = i0; i < quads; i += stride)
+    reinterpret_cast<float4*>(grad + L.b4)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (long i = L.b4 + 4 * quads + i0; i < L.total; i += stride) grad[i] = 0.0f;
+  if (i0 < 2) sums[i0] = 0.0;
 }
 
 __global__ void k_init_params(float* th, Layout L, uint64_t seed) {
@@ -767,12 +762,10 @@ using namespace racer;
 
 struct SurrogateActs {  // activation buffers and tensor maps for one row count M
   int M = 0;
-  bf16 *x = nullptr, *xf = nullptr, *h1s = nullptr, *h2s = nullptr, *h3s = nullptr;
-  bf16 *h1f = nullptr, *h2f = nullptr, *h3f = nullptr;
-  bf16 *g4s = nullptr, *g4f = nullptr, *g3s = nullptr, *g3f = nullptr, *g2s = nullptr, *g2f = nullptr,
-       *g1f = nullptr, *g1s = nullptr;
-  CUtensorMap tx, th1, th2, th3, tg4s, tg3s, tg2s, tg1s;    // A operands (M rows)
-  CUtensorMap tg4f, tg3f, tg2f, tg1f, th3f, th2f, th1f, txf;  // weight-gradient operands (K = M)
+  bf16 *x = nullptr, *h1s = nullptr, *h2s = nullptr, *h3s = nullptr;
+  bf16 *g4s = nullptr, *g3s = nullptr, *g2s = nullptr, *g1s = nullptr;
+  CUtensorMap tx, th1, th2, th3, tg4s, tg3s, tg2s, tg1s;      // A operands (M rows)
+  CUtensorMap wg4, wg3, wg2, wg1, wh3, wh2, wh1, wx;          // the same as weight-gradient operands (K = M)
 };
 
 struct racer_surrogate {
@@ -787,10 +780,11 @@ struct racer_surrogate {
   bf16 *w1b = nullptr, *w2b = nullptr, *w3b = nullptr, *w4b = nullptr, *w2t = nullptr, *w3t = nullptr,
        *w4t = nullptr, *w1t = nullptr;
   CUtensorMap tw1, tw2, tw3, tw4, tw2t, tw3t, tw4t, tw1t;  // B operands
-  // world frame: grid geometry, world outputs of a training batch (FP32 [batch, npad]), the
-  // input gradient (FP32 [batch, 64]), world profiles of a batch and of the sim's cars (FP16)
+  // world frame: grid geometry, a training batch's labels by world sample (FP32 [batch, npad]) and
+  // first world samples, the input gradient (FP32 [batch, 64]), world profiles of a batch and of the sim's cars (FP16)
   GridGeom gg{};
-  float* wy = nullptr;
+  float* wtarget = nullptr;
+  int* wk0 = nullptr;
   float* dx = nullptr;
   __half* wbatch = nullptr;
   __half* wout = nullptr;
@@ -854,28 +848,21 @@ int make_acts(racer_surrogate* s, SurrogateActs* a, int M, bool training) {
     racer_host::set_error("surrogate: the training batch must be a multiple of 8");
     return 1;
   }
-  if ((rc = salloc(&a->xf, (size_t)NIN * M)) || (rc = salloc(&a->h1f, (size_t)H * M)) ||
-      (rc = salloc(&a->h2f, (size_t)H * M)) || (rc = salloc(&a->h3f, (size_t)H * M)) ||
-      (rc = salloc(&a->g4s, (size_t)M * NP)) || (rc = salloc(&a->g4f, (size_t)NP * M)) ||
-      (rc = salloc(&a->g3s, (size_t)M * H)) || (rc = salloc(&a->g3f, (size_t)H * M)) ||
-      (rc = salloc(&a->g2s, (size_t)M * H)) || (rc = salloc(&a->g2f, (size_t)H * M)) ||
-      (rc = salloc(&a->g1f, (size_t)H * M)) || (rc = salloc(&a->g1s, (size_t)M * H)))
+  if ((rc = salloc(&a->g4s, (size_t)M * NP)) || (rc = salloc(&a->g3s, (size_t)M * H)) ||
+      (rc = salloc(&a->g2s, (size_t)M * H)) || (rc = salloc(&a->g1s, (size_t)M * H)))
     return rc;
   if ((rc = make_tmap_bf16(&a->tg4s, a->g4s, M, NP, NP, 128)) || (rc = make_tmap_bf16(&a->tg3s, a->g3s, M, H, H, 128)) ||
       (rc = make_tmap_bf16(&a->tg2s, a->g2s, M, H, H, 128)) || (rc = make_tmap_bf16(&a->tg1s, a->g1s, M, H, H, 128)) ||
-      (rc = make_tmap_bf16(&a->tg4f, a->g4f, NP, M, M, 128)) ||
-      (rc = make_tmap_bf16(&a->tg3f, a->g3f, H, M, M, 128)) || (rc = make_tmap_bf16(&a->tg2f, a->g2f, H, M, M, 128)) ||
-      (rc = make_tmap_bf16(&a->tg1f, a->g1f, H, M, M, 128)) || (rc = make_tmap_bf16(&a->th3f, a->h3f, H, M, M, 256)) ||
-      (rc = make_tmap_bf16(&a->th2f, a->h2f, H, M, M, 256)) || (rc = make_tmap_bf16(&a->th1f, a->h1f, H, M, M, 256)) ||
-      (rc = make_tmap_bf16(&a->txf, a->xf, NIN, M, M, 64)))
+      (rc = make_tmap_bf16(&a->wg4, a->g4s, M, NP, NP, 64)) || (rc = make_tmap_bf16(&a->wg3, a->g3s, M, H, H, 64)) ||
+      (rc = make_tmap_bf16(&a->wg2, a->g2s, M, H, H, 64)) || (rc = make_tmap_bf16(&a->wg1, a->g1s, M, H, H, 64)) ||
+      (rc = make_tmap_bf16(&a->wh3, a->h3s, M, H, H, 64)) || (rc = make_tmap_bf16(&a->wh2, a->h2s, M, H, H, 64)) ||
+      (rc = make_tmap_bf16(&a->wh1, a->h1s, M, H, H, 64)) || (rc = make_tmap_bf16(&a->wx, a->x, M, NIN, NIN, 64)))
     return rc;
   return 0;
 }
 
 void free_acts(SurrogateActs* a) {
-  for (bf16* p : {a->x, a->xf, a->h1s, a->h2s, a->h3s, a->h1f, a->h2f, a->h3f, a->g4s, a->g4f, a->g3s, a->g3f, a->g2s,
-                  a->g2f, a->g1f, a->g1s})
-    cudaFree(p);
+  for (bf16* p : {a->x, a->h1s, a->h2s, a->h3s, a->g4s, a->g3s, a->g2s, a->g1s}) cudaFree(p);
 }
 
 #define SURR_CHECK(expr)                                                                  \
@@ -888,16 +875,15 @@ void free_acts(SurrogateActs* a) {
   } while (0)
 
 // Forward of M rows already featurised in a->x; the last layer uses `out` (inference).
-int forward(racer_surrogate* s, SurrogateActs* a, bool training, const EpiInfer* out) {
+int forward(racer_surrogate* s, SurrogateActs* a, const EpiInfer* out) {
   const int H = s->L.H, M = a->M;
   const float* th = s->theta;
   cudaStream_t st = s->st;
-  SURR_CHECK(gemm_launch<256>(a->tx, s->tw1, M, H, 1, 1, EpiTanhOut{a->h1s, H, training ? a->h1f : nullptr, M, nullptr, M, H},
-                              s->err, st));
+  SURR_CHECK(gemm_launch<256>(a->tx, s->tw1, M, H, 1, 1, EpiTanhOut{a->h1s, H, nullptr, M, H}, s->err, st));
   SURR_CHECK(gemm_launch<256>(a->th1, s->tw2, M, H, H / 64, 1,
-                              EpiTanhOut{a->h2s, H, training ? a->h2f : nullptr, M, th + s->L.b2, M, H}, s->err, st));
+                              EpiTanhOut{a->h2s, H, th + s->L.b2, M, H}, s->err, st));
   SURR_CHECK(gemm_launch<256>(a->th2, s->tw3, M, H, H / 64, 1,
-                              EpiTanhOut{a->h3s, H, training ? a->h3f : nullptr, M, th + s->L.b3, M, H}, s->err, st));
+                              EpiTanhOut{a->h3s, H, th + s->L.b3, M, H}, s->err, st));
   if (out) SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, M, s->L.beams, H / 64, 1, *out, s->err, st));
   return 0;
 }
@@ -906,7 +892,7 @@ int forward(racer_surrogate* s, SurrogateActs* a, bool training, const EpiInfer*
 // `ray` [2, M]: world profiles into wout [M, npad] (FP16); minr (optional)
 // gets each row's smallest predicted range.
 int world_profiles(racer_surrogate* s, SurrogateActs* a, const float4* ray, __half* wout, unsigned* minr) {
-  int rc = forward(s, a, false, nullptr);
+  int rc = forward(s, a, nullptr);
   if (rc) return rc;
   const int H = s->L.H, M = a->M;
   EpiWorldInfer epi{wout, s->L.npad, s->theta + s->L.b4, M, s->L.nout, ray, s->L.beams, minr};
@@ -929,7 +915,7 @@ int world_rotate(racer_surrogate* s, const __half* wout, const float4* ray, int 
   return 0;
 }
 
-// BN must equal the row box of tb's tensor map (256 for the hidden activations, 64 for the inputs).
+// grad[off ..] = G^T H over the batch: G [batch, M], H [batch, N] (MN-major operands).
 template <int BN>
 int wgrad(racer_surrogate* s, const CUtensorMap& ta, const CUtensorMap& tb, int Mpad, int Mreal, int N, long off) {
   const int kblocks = (s->batch + 63) / 64;
@@ -942,23 +928,22 @@ int wgrad(racer_surrogate* s, const CUtensorMap& ta, const CUtensorMap& tb, int 
     return 1;
   }
   EpiSplitF32 epi{s->scratch, (long)Mpad * N, Mpad, N};
-  SURR_CHECK(gemm_launch<BN>(ta, tb, Mpad, N, kblocks, splits, epi, s->err, s->st));
+  SURR_CHECK((gemm_launch<BN, EpiSplitF32, true>(ta, tb, Mpad, N, kblocks, splits, epi, s->err, s->st)));
   long count = (long)Mreal * N;
-  k_reduce_splits<<<(unsigned)((count + 255) / 256), 256, 0, s->st>>>(s->scratch, splits, (long)Mpad * N, N, Mreal,
-                                                                       s->grad + off);
+  k_reduce_splits<<<(unsigned)((count / 4 + 127) / 128), 128, 0, s->st>>>(s->scratch, splits, (long)Mpad * N, count,
+                                                                          s->grad + off);
   SURR_CHECK(cudaGetLastError());
   return 0;
 }
 
-// Encoded inputs of `count` ray frames (sample-major x; feature-major xf if given).
-int featurise(racer_surrogate* s, const float4* ray, int count, bf16* x, bf16* xf, cudaStream_t st) {
+// Encoded inputs x [count, 64] of `count` ray frames.
+int featurise(racer_surrogate* s, const float4* ray, int count, bf16* x, cudaStream_t st) {
   if (s->L.world)
-    k_features_world<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, s->gg, s->theta + s->L.g, s->L.nout, x,
-                                                          xf);
+    k_features_world<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, s->gg, s->theta + s->L.g, s->L.nout, x);
   else if (s->L.grid)
-    k_features_cargrid<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, s->gg, s->theta + s->L.g, x, xf);
+    k_features_cargrid<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, s->gg, s->theta + s->L.g, x);
   else
-    k_features<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, x, xf);
+    k_features<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, x);
   SURR_CHECK(cudaGetLastError());
   return 0;
 }
@@ -966,64 +951,59 @@ int featurise(racer_surrogate* s, const float4* ray, int count, bf16* x, bf16* x
 // Labels and features for batch rows taken from the pose set starting at `first`.
 // Frames, exact labels and encoded inputs of the batch at pose `first`; with
 // `cached`, the labels come from (or go to) the label cache of the pose set.
-int prepare(racer_surrogate* s, SurrogateActs* a, long first, bool cached = false) {
+// *labels gets the labels [beams, batch]: their place in the cache, or the rows of s->label.
+int prepare(racer_surrogate* s, SurrogateActs* a, long first, const float** labels, bool cached = false) {
   racer_sim* sim = s->sim;
   const int B = a->M;
   const float4* poses = s->poses + first;
   launch_pose_frames(sim->t, poses, B, s->ray, s->st);
   const long b = first / B;
   const size_t block = (size_t)sim->beams * B;
-  float* slot = cached && s->lcache && first % B == 0 ? s->lcache + b * block : nullptr;
-  if (slot && s->lcached[b]) {
-    SURR_CHECK(cudaMemcpyAsync(s->label + 4L * B, slot, block * sizeof(float), cudaMemcpyDeviceToDevice, s->st));
-  } else {
-    launch_lidar(sim->t, s->ray, s->label, B, sim->beams, sim->beam_dir, nullptr, s->st);
-    if (slot) {
-      SURR_CHECK(cudaMemcpyAsync(slot, s->label + 4L * B, block * sizeof(float), cudaMemcpyDeviceToDevice, s->st));
-      s->lcached[b] = 1;
-    }
+  float* slot = cached && s->lcache && first % B == 0 ? s->lcache + b * block : s->label + 4L * B;
+  const bool keep = slot != s->label + 4L * B;  // traced into the cache, and read there from then on
+  if (!keep || !s->lcached[b]) {
+    launch_lidar(sim->t, s->ray, slot - 4L * B, B, sim->beams, sim->beam_dir, nullptr, s->st);  // writes rows 4.. only
+    if (keep) s->lcached[b] = 1;
   }
-  return featurise(s, s->ray, B, a->x, a->xf, s->st);
+  *labels = slot;
+  return featurise(s, s->ray, B, a->x, s->st);
 }
 
 // Gradient of the mean squared error over the batch into s->grad; loss sums into s->sums.
-int gradient(racer_surrogate* s, long first) {
+int gradient(racer_surrogate* s, long first, const float** labels) {
   SurrogateActs* a = &s->train;
   const int H = s->L.H, B = a->M, NP = s->L.npad, beams = s->L.beams;
-  int rc = prepare(s, a, first, true);
+  int rc = prepare(s, a, first, labels, true);
   if (rc) return rc;
-  SURR_CHECK(cudaMemsetAsync(s->grad + s->L.b2, 0, H * sizeof(float), s->st));
-  SURR_CHECK(cudaMemsetAsync(s->grad + s->L.b3, 0, H * sizeof(float), s->st));
   const int nout = s->L.nout;
-  SURR_CHECK(cudaMemsetAsync(s->grad + s->L.b4, 0, nout * sizeof(float), s->st));
-  SURR_CHECK(cudaMemsetAsync(s->sums, 0, 2 * sizeof(double), s->st));
-  if (s->L.grid)
-    SURR_CHECK(cudaMemsetAsync(s->grad + s->L.g, 0, (s->L.total - s->L.g) * sizeof(float), s->st));
-  if ((rc = forward(s, a, true, nullptr))) return rc;
+  k_zero_sums<<<device_sms(), 256, 0, s->st>>>(s->grad, s->L, s->sums);
+  SURR_CHECK(cudaGetLastError());
+  if ((rc = forward(s, a, nullptr))) return rc;
   const float scale = 2.0f / ((float)B * (float)beams);
+  LossSums losses;
+  losses.sums = s->sums;
   if (s->L.world) {
-    SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, EpiWorldTrain{s->wy, NP, s->theta + s->L.b4, B, nout},
-                                s->err, s->st));
-    k_world_loss<<<dim3(B / 128, NP / 64), 128, 0, s->st>>>(s->wy, s->label + 4L * B, s->ray, B, beams, nout, NP,
-                                                            scale, s->huber, a->g4s, a->g4f, s->grad + s->L.b4,
-                                                            s->sums);
+    k_world_targets<<<dim3((B + 31) / 32, (beams + 31) / 32), 256, 0, s->st>>>(*labels, s->ray, B, beams, nout,
+                                                                               NP, s->wtarget, s->wk0);
     SURR_CHECK(cudaGetLastError());
+    EpiLoss<true> loss{s->wtarget, 0, s->wk0, beams, s->theta + s->L.b4, B, nout, scale, a->g4s, NP,
+                       s->grad + s->L.b4, s->huber, losses};
+    SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, loss, s->err, s->st));
   } else {
-    EpiLoss loss{s->label + 4L * B, B, s->theta + s->L.b4, B, beams, scale,
-                 a->g4s, NP, a->g4f, B, s->grad + s->L.b4, s->sums, NP, s->huber};
+    EpiLoss<false> loss{*labels, B, nullptr, beams, s->theta + s->L.b4, B, beams, scale, a->g4s, NP,
+                        s->grad + s->L.b4, s->huber, losses};
     SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, loss, s->err, s->st));
   }
   SURR_CHECK(gemm_launch<256>(a->tg4s, s->tw4t, B, H, NP / 64, 1,
-                              EpiDTanh{a->h3s, H, a->g3s, H, a->g3f, B, s->grad + s->L.b3, B, H}, s->err, s->st));
+                              EpiDTanh{a->h3s, H, a->g3s, H, s->grad + s->L.b3, B, H}, s->err, s->st));
   SURR_CHECK(gemm_launch<256>(a->tg3s, s->tw3t, B, H, H / 64, 1,
-                              EpiDTanh{a->h2s, H, a->g2s, H, a->g2f, B, s->grad + s->L.b2, B, H}, s->err, s->st));
-  SURR_CHECK(gemm_launch<256>(a->tg2s, s->tw2t, B, H, H / 64, 1,
-                              EpiDTanh{a->h1s, H, s->L.grid ? a->g1s : nullptr, H, a->g1f, B, nullptr, B, H}, s->err,
+                              EpiDTanh{a->h2s, H, a->g2s, H, s->grad + s->L.b2, B, H}, s->err, s->st));
+  SURR_CHECK(gemm_launch<256>(a->tg2s, s->tw2t, B, H, H / 64, 1, EpiDTanh{a->h1s, H, a->g1s, H, nullptr, B, H}, s->err,
                               s->st));
-  if ((rc = wgrad<256>(s, a->tg4f, a->th3f, NP, nout, H, s->L.w4))) return rc;
-  if ((rc = wgrad<256>(s, a->tg3f, a->th2f, H, H, H, s->L.w3))) return rc;
-  if ((rc = wgrad<256>(s, a->tg2f, a->th1f, H, H, H, s->L.w2))) return rc;
-  if ((rc = wgrad<64>(s, a->tg1f, a->txf, H, H, NIN, s->L.w1))) return rc;
+  if ((rc = wgrad<256>(s, a->wg4, a->wh3, NP, nout, H, s->L.w4))) return rc;
+  if ((rc = wgrad<256>(s, a->wg3, a->wh2, H, H, H, s->L.w3))) return rc;
+  if ((rc = wgrad<256>(s, a->wg2, a->wh1, H, H, H, s->L.w2))) return rc;
+  if ((rc = wgrad<64>(s, a->wg1, a->wx, H, H, NIN, s->L.w1))) return rc;
   if (s->L.grid) {  // dL/df = g1 W1, then onto the grids
     SURR_CHECK(gemm_launch<64>(a->tg1s, s->tw1t, B, NIN, H / 64, 1, EpiRowF32{s->dx, NIN, B, NIN}, s->err, s->st));
     k_grid_grad<<<B / 128, 128, 0, s->st>>>(s->ray, B, s->gg, s->dx, s->grad + s->L.g);
@@ -1111,7 +1091,8 @@ int racer_surrogate_create_frame(racer_sim* sim, int hidden, int batch, uint64_t
   int rc = 0;
   if ((L.grid && ((rc = salloc(&s->w1t, (size_t)NIN * H)) || (rc = salloc(&s->dx, (size_t)batch * NIN)) ||
                    (rc = make_tmap_bf16(&s->tw1t, s->w1t, NIN, H, H, 64)))) ||
-      (L.world && ((rc = salloc(&s->wy, (size_t)batch * NP)) || (rc = salloc(&s->wbatch, (size_t)batch * NP))))) {
+      (L.world && ((rc = salloc(&s->wtarget, (size_t)batch * NP)) || (rc = salloc(&s->wk0, (size_t)batch)) ||
+                   (rc = salloc(&s->wbatch, (size_t)batch * NP))))) {
     racer_surrogate_destroy(s);
     return rc;
   }
@@ -1166,7 +1147,7 @@ int racer_surrogate_create_frame(racer_sim* sim, int hidden, int batch, uint64_t
 
 int racer_surrogate_destroy(racer_surrogate* s) {
   if (!s) return 0;
-  for (void* p : {(void*)s->w1t, (void*)s->wy, (void*)s->dx, (void*)s->wbatch, (void*)s->wout})
+  for (void* p : {(void*)s->w1t, (void*)s->wtarget, (void*)s->wk0, (void*)s->dx, (void*)s->wbatch, (void*)s->wout})
     cudaFree(p);
   for (void* p : {(void*)s->theta, (void*)s->grad, (void*)s->m1, (void*)s->m2, (void*)s->w1b, (void*)s->w2b,
                   (void*)s->w3b, (void*)s->w4b, (void*)s->w2t, (void*)s->w3t, (void*)s->w4t, (void*)s->cells,
@@ -1249,7 +1230,7 @@ int racer_surrogate_batch_predict(racer_surrogate* s, float* pred) {
     if (!rc) rc = world_rotate(s, s->wbatch, s->ray, B, pred, B, s->st);
   } else {
     EpiInfer inf{pred, B, s->theta + s->L.b4, B, s->L.beams, nullptr};
-    rc = forward(s, a, false, &inf);
+    rc = forward(s, a, &inf);
   }
   if (rc) return rc;
   RACER_TRY(cudaStreamSynchronize(s->st));
@@ -1381,9 +1362,10 @@ int racer_surrogate_gradient(racer_surrogate* s, long first, float* mse, float* 
     racer_host::set_error("racer_surrogate_gradient: set poses first; the batch must lie inside the pose set");
     return 1;
   }
-  if (int rc = gradient(s, first)) return rc;
+  const float* labels = nullptr;
+  if (int rc = gradient(s, first, &labels)) return rc;
   if (label_dev_out)
-    RACER_TRY(cudaMemcpyAsync(label_dev_out, s->label + 4L * s->batch, (size_t)s->L.beams * s->batch * sizeof(float),
+    RACER_TRY(cudaMemcpyAsync(label_dev_out, labels, (size_t)s->L.beams * s->batch * sizeof(float),
                               cudaMemcpyDeviceToDevice, s->st));
   double sums[2];
   RACER_TRY(cudaMemcpyAsync(sums, s->sums, sizeof sums, cudaMemcpyDeviceToHost, s->st));
@@ -1401,7 +1383,8 @@ int racer_surrogate_train(racer_surrogate* s, int steps, float lr, float* last_m
   const int per_epoch = s->npose / s->batch;
   for (int k = 0; k < steps; ++k) {
     long first = (long)(s->step % per_epoch) * s->batch;
-    if (int rc = gradient(s, first)) return rc;
+    const float* labels = nullptr;
+    if (int rc = gradient(s, first, &labels)) return rc;
     s->step += 1;
     const float frac = (float)k / (float)steps;
     const float rate = lr * (0.01f + 0.99f * 0.5f * (1.0f + cosf(3.14159265f * frac)));
@@ -1456,16 +1439,17 @@ int racer_surrogate_evaluate(racer_surrogate* s, int batches, uint64_t seed, flo
   SurrogateActs* a = &s->train;
   const int B = s->batch;
   for (int k = 0; k < batches && !rc; ++k) {
-    if ((rc = prepare(s, a, (long)k * B))) break;
+    const float* labels = nullptr;
+    if ((rc = prepare(s, a, (long)k * B, &labels))) break;
     if (s->L.world) {
       if ((rc = world_profiles(s, a, s->ray, s->wbatch, nullptr)) ||
           (rc = world_rotate(s, s->wbatch, s->ray, B, s->pred, B, s->st)))
         break;
     } else {
       EpiInfer inf{s->pred, B, s->theta + s->L.b4, B, s->L.beams, nullptr};
-      if ((rc = forward(s, a, false, &inf))) break;
+      if ((rc = forward(s, a, &inf))) break;
     }
-    k_compare<<<296, 256, 0, s->st>>>(s->pred, s->label + 4L * B, (long)s->L.beams * B, s->sums + 2, s->maxbits,
+    k_compare<<<296, 256, 0, s->st>>>(s->pred, labels, (long)s->L.beams * B, s->sums + 2, s->maxbits,
                                       s->over);
   }
   cudaFree(s->poses);
@@ -1577,7 +1561,7 @@ int surrogate_lidar(racer_surrogate* s, racer_sim* sim, float* obs, bool audit, 
                     const int64_t* step_base, int64_t step_add) {
   const int n = sim->n, beams = sim->beams;
   SurrogateActs* a = &s->infer;
-  if (int rc = featurise(s, sim->ray, n, a->x, nullptr, st)) return rc;
+  if (int rc = featurise(s, sim->ray, n, a->x, st)) return rc;
   SURR_CHECK(cudaMemsetAsync(s->minr, 0x7f, (size_t)n * sizeof(unsigned), st));
   // on an audit step the prediction goes to the scratch rows and the exact tracer writes obs
   float* pred = audit ? s->exact + 4L * n : obs + 4L * n;
@@ -1595,7 +1579,7 @@ int surrogate_lidar(racer_surrogate* s, racer_sim* sim, float* obs, bool audit, 
       rc = world_profiles(s, a, sim->ray, s->wout, s->minr);
     } else {
       EpiInfer inf{pred, n, s->theta + s->L.b4, n, beams, s->minr};
-      rc = forward(s, a, false, &inf);
+      rc = forward(s, a, &inf);
     }
     s->st = keep;
     if (rc) return rc;
