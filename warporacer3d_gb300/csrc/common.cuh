@@ -105,6 +105,25 @@ inline int device_sms() {
   return cache[dev];
 }
 
+#if defined(__CUDACC__)
+// Programmatic dependent launch: a kernel launched with `launch_early` becomes resident once every block of the kernel
+// before it in the stream has called early_start (or ended) and must call it itself before it touches memory: it waits
+// until that kernel has completed. Hides a launch's latency behind its predecessor.
+__device__ __forceinline__ void early_start() {
+  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t launch_early(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at, cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+#endif
+
 // Per-device one-time set-up (kernel attributes such as the dynamic shared
 // memory limit belong to each device's context): runs `setup` unless it has
 // already succeeded on the current device, as recorded in `mask`.

@@ -519,6 +519,7 @@ __device__ __forceinline__ void advance_car(const TrackDev& t, float* s, const f
 __global__ void k_advance(const __grid_constant__ Segments g, float* s, const float* act, float* reward, float* done,
                           float* obs, int n, int beams, float4* ray, double* eval_reward, int* eval_crash, int c0,
                           int c1) {
+  early_start();
   const int i = c0 + (int)(blockIdx.x * blockDim.x + threadIdx.x);
   if (i >= c1) return;
   const int k = segment_of(g, i);
@@ -685,6 +686,7 @@ __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
     k_lidar_track(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0, int c1,
                   int beams, const float2* __restrict__ beam_dir, int* iters, const int* __restrict__ list,
                   const int* list_count) {
+  early_start();
   const int beam = blockIdx.y * 32 + (threadIdx.x & 31);
   if (beam >= beams) return;
   if (LIST) {  // only the listed cars (surrogate fallback), grid-stride over the list
@@ -708,6 +710,7 @@ template <int LAYERS, int CARS, bool WIDE>
 __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
     k_lidar_flat(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0,
                  unsigned items, int beams, const float2* __restrict__ beam_dir, int* iters) {
+  early_start();
   const unsigned item = (blockIdx.x * CARS + (threadIdx.x >> 5)) * 32u + (threadIdx.x & 31);
   if (item >= items) return;
   const unsigned car = item / (unsigned)beams;
@@ -750,6 +753,7 @@ __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
     k_lidar_segments(const __grid_constant__ Segments g, const __grid_constant__ LidarGrid lg,
                      const float4* __restrict__ ray, float* obs, int n, int beams,
                      const float2* __restrict__ beam_dir, int* iters) {
+  early_start();
   const int beam = blockIdx.y * 32 + (threadIdx.x & 31);
   if (beam >= beams) return;
   int j = 0;
@@ -947,8 +951,8 @@ void launch_advance(const Segments& g, float* state, const float* actions, float
                     int c1) {
   if (c1 < 0) c1 = n;
   if (c1 <= c0) return;
-  k_advance<<<(c1 - c0 + 127) / 128, 128, 0, st>>>(g, state, actions, reward, done, obs, n, beams, ray, eval_reward,
-                                                   eval_crash, c0, c1);
+  launch_early(k_advance, dim3((c1 - c0 + 127) / 128), 128, 0, st, g, state, actions, reward, done, obs, n, beams, ray,
+               eval_reward, eval_crash, c0, c1);
 }
 
 
@@ -985,32 +989,37 @@ static LidarGrid lidar_grid(const Segments& g, const LidarShape& shape) {
 // without (4352 blocks, one of 16 rollout chains: 6.45 ms a rollout against 6.88).
 constexpr long BIG_LIDAR = 1 << 18;
 template <class... P, class... A>
-static void lidar_launch(void (*k)(P...), dim3 grid, unsigned threads, cudaStream_t st, A... args) {
+static void lidar_launch(void (*k)(P...), dim3 grid, unsigned threads, cudaStream_t st, bool early, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.stream = st;
   cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-  at.val.sharedMemCarveout = 14;  // per cent of 228 KB
-  cfg.attrs = &at, cfg.numAttrs = (long)grid.x * grid.y >= BIG_LIDAR ? 1 : 0;
+  if ((long)grid.x * grid.y >= BIG_LIDAR) {
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = 14;  // per cent of 228 KB
+  } else {
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = early;
+  }
+  cfg.attrs = &at, cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
 template <int LAYERS, int CARS, bool WIDE>
 static void lidar_track(const TrackDev& t, int max_iters, const float4* ray, float* obs, int n, int c0, int c1,
-                        int beams, const float2* beam_dir, int* iters, cudaStream_t st, bool flat = false) {
+                        int beams, const float2* beam_dir, int* iters, cudaStream_t st, bool flat, bool early) {
   const long items = (long)(c1 - c0) * beams;
   // Warps across car boundaries where asked for, and where a car's last warp would leave more than a twelfth of the
   // lanes idle: 108 beams (16%) at 16384 cars 58.0 us against 62.4; at 181 (6%) and 300 (6%) beams either takes as long.
   const int lanes = (beams + 31) / 32 * 32;
   if ((flat || (lanes - beams) * 12 > lanes) && items > 0 && items < (1L << 31)) {
     const unsigned blocks = (unsigned)((items + 32 * CARS - 1) / (32 * CARS));
-    lidar_launch(k_lidar_flat<LAYERS, CARS, WIDE>, dim3(blocks), CARS * 32, st, t, max_iters, ray, obs, n, c0,
+    lidar_launch(k_lidar_flat<LAYERS, CARS, WIDE>, dim3(blocks), CARS * 32, st, early, t, max_iters, ray, obs, n, c0,
                  (unsigned)items, beams, beam_dir, iters);
     return;
   }
   dim3 grid((c1 - c0 + CARS - 1) / CARS, (beams + 31) / 32);
   if (grid.x == 0) return;
-  lidar_launch(k_lidar_track<LAYERS, CARS, WIDE, false>, grid, CARS * 32, st, t, max_iters, ray, obs, n, c0, c1, beams,
+  lidar_launch(k_lidar_track<LAYERS, CARS, WIDE, false>, grid, CARS * 32, st, early, t, max_iters, ray, obs, n, c0, c1, beams,
                beam_dir, iters, (const int*)nullptr, (const int*)nullptr);
 }
 
@@ -1028,7 +1037,8 @@ static void lidar_dynamic(const TrackDev& t, int max_iters, const float4* ray, f
 
 template <int CARS, bool WIDE>
 static void lidar_segment(const Segments& g, int k, const float4* ray, float* obs, int n, int beams,
-                          const float2* beam_dir, int* iters, cudaStream_t st, const LidarShape& shape) {
+                          const float2* beam_dir, int* iters, cudaStream_t st, const LidarShape& shape,
+                          bool early = false) {
   const TrackDev& t = g.t[k];
   const int c0 = g.car0[k], c1 = g.car0[k + 1];
   if (shape.dynamic && shape.counters) {
@@ -1043,23 +1053,23 @@ static void lidar_segment(const Segments& g, int k, const float4* ray, float* ob
   }
   const bool flat = shape.flat == 1;
   if (t.layers == 1)
-    lidar_track<1, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat);
+    lidar_track<1, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);
   else if (t.layers == 2)
-    lidar_track<2, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat);
+    lidar_track<2, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);
   else
-    lidar_track<0, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat);
+    lidar_track<0, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);
 }
 
 template <int CARS, bool WIDE>
 static void lidar_shape(const Segments& g, const LidarShape& shape, const float4* ray, float* obs, int n, int beams,
                         const float2* beam_dir, int* iters, cudaStream_t st) {
   if (g.count == 1) {
-    lidar_segment<CARS, WIDE>(g, 0, ray, obs, n, beams, beam_dir, iters, st, shape);
+    lidar_segment<CARS, WIDE>(g, 0, ray, obs, n, beams, beam_dir, iters, st, shape, true);
     return;
   }
   const LidarGrid lg = lidar_grid(g, shape);
   dim3 grid(lg.block0[g.count], (beams + 31) / 32);
-  lidar_launch(k_lidar_segments<CARS, WIDE>, grid, CARS * 32, st, g, lg, ray, obs, n, beams, beam_dir, iters);
+  lidar_launch(k_lidar_segments<CARS, WIDE>, grid, CARS * 32, st, true, g, lg, ray, obs, n, beams, beam_dir, iters);
 }
 
 bool lidar_shape_ok(const LidarShape& shape) {
@@ -1102,14 +1112,14 @@ void launch_lidar_cars(const Segments& g, const LidarShape& shape, int c0, int c
   if (g.count != 1 || c1 <= c0) return;
   const TrackDev& t = g.t[0];
   const bool wide = shape.wide == 1;
-  const bool flat = shape.flat == 1;
+  const bool flat = shape.flat == 1, early = false;  // one chain's waiting blocks would hold another's places
 #define RACER_LIDAR_CARS(CARS, WIDE)                                                                         \
   if (t.layers == 1)                                                                                          \
-    lidar_track<1, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat);   \
+    lidar_track<1, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);   \
   else if (t.layers == 2)                                                                                     \
-    lidar_track<2, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat);   \
+    lidar_track<2, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);   \
   else                                                                                                        \
-    lidar_track<0, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat);
+    lidar_track<0, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);
   if (shape.cars == 2) {
     if (wide) { RACER_LIDAR_CARS(2, true) } else { RACER_LIDAR_CARS(2, false) }
   } else if (shape.cars == 8) {
