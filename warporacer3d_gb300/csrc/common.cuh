@@ -107,20 +107,29 @@ inline int device_sms() {
 
 #if defined(__CUDACC__)
 // Programmatic dependent launch: a kernel launched with `launch_early` becomes resident once every block of the kernel
-// before it in the stream has called early_start (or ended) and must call it itself before it touches memory: it waits
-// until that kernel has completed. Hides a launch's latency behind its predecessor.
+// before it in the stream has called early_next (or ended), and must call early_wait, which returns once that kernel
+// has completed, before it touches memory that another kernel does. Hides a launch's latency, and what a kernel sets up
+// for itself, behind its predecessor. Both calls do nothing in a kernel launched otherwise.
+__device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void early_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void early_start() {
-  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
+  early_next();
+  early_wait();
 }
 template <class... P, class... A>
-cudaError_t launch_early(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+cudaError_t launch_early_if(bool early, void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st,
+                            A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
+  at.val.programmaticStreamSerializationAllowed = early;
   cfg.attrs = &at, cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+template <class... P, class... A>
+cudaError_t launch_early(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A... args) {
+  return launch_early_if(true, k, grid, threads, smem, st, args...);
 }
 #endif
 

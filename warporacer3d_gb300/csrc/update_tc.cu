@@ -156,6 +156,10 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
       for (int e = tid; e < bytes / 16; e += C::THREADS) reinterpret_cast<uint4*>(smem + off)[e] = __ldg(s + e);
     };
     const int w0_bytes = (in + 63) / 64 * W_BYTES;
+    for (int e = tid; e < TILE_BYTES / 16; e += C::THREADS)  // unit 0 of every sample is 1
+      reinterpret_cast<uint4*>(smem + C::ONE)[e] =
+          make_uint4((e & 7) == ((e >> 3) & 7) ? tc::pack_bf16(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
+    early_wait();  // theta and its images are the last minibatch's
     copy(C::W0, a.pack, w0_bytes);
     copy(C::W1, a.pack + w0_bytes, 2 * W_BYTES);
     copy(C::W2, a.pack + w0_bytes + 2 * W_BYTES, 2 * 16 * 128);
@@ -164,13 +168,11 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
       const float* w = a.theta + w2 + tid;
       w2f[tid] = make_float4(__ldg(w), __ldg(w + HA), __ldg(w + 2 * HA), 0.0f);
     }
-    for (int e = tid; e < TILE_BYTES / 16; e += C::THREADS)  // unit 0 of every sample is 1
-      reinterpret_cast<uint4*>(smem + C::ONE)[e] =
-          make_uint4((e & 7) == ((e >> 3) & 7) ? tc::pack_bf16(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
   }
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
   __syncthreads();
+  early_next();  // not before the TMEM is allocated: a CTA that waits for this kernel must not hold what this one needs
   tc::tc_fence_after();
   const uint32_t tmem = *tslot + ctx * C::COLS;
   const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
@@ -421,6 +423,7 @@ __global__ void __launch_bounds__(RED_W * 32) k_update_reduce(const float* __res
                                                              float* grad, double* squares, float* stats) {
   __shared__ float sh[32][RED_W + 1];
   __shared__ double sq[32];
+  early_start();
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
   float g = 0.0f;
   if (blockIdx.x + 1 < gridDim.x) {
@@ -467,6 +470,7 @@ __global__ void __launch_bounds__(256) k_update_adam(int in, int parts, const do
                                                      const float* __restrict__ grad, float* first, float* second,
                                                      uint8_t* pack, bf16* w1t) {
   __shared__ double sh[256];
+  early_start();
   double q = 0.0;
   for (int k = threadIdx.x; k < parts; k += 256) q += squares[k];
   sh[threadIdx.x] = q;
@@ -575,11 +579,12 @@ cudaError_t launch_update_minibatch(UpdateWork* w, int m, const CUtensorMap& xma
   const int weights = H * w->in + H * HA + OUT * HA, blocks = reduce_blocks(weights);
   const TileArgs a{w->samples + (size_t)m * 5 * w->batch, w->in,   w->batch, w->range, w->ranges, theta, pack, w->w1t,
                    stats + ST_ADV,                        w->part, w->sums,  dump,     err};
-  k_update_tiles<<<w->ctas, UpdateCfg::THREADS, UpdateCfg::SMEM, st>>>(xmap, a);
-  k_update_reduce<<<blocks, RED_W * 32, 0, st>>>(w->part, w->ranges, w->sums, w->ctas, weights, grad, w->squares,
-                                                 stats);
-  k_update_adam<<<(weights + 2 + 255) / 256, 256, 0, st>>>(w->in, blocks, w->squares, c12, stats, theta, grad, first,
-                                                           second, pack, reinterpret_cast<bf16*>(w->w1t));
+  // Early, each behind the kernel before it: 81.0 us a minibatch against 81.9 (16 x 65536 samples of 108 inputs).
+  launch_early(k_update_tiles, dim3(w->ctas), UpdateCfg::THREADS, UpdateCfg::SMEM, st, xmap, a);
+  launch_early(k_update_reduce, dim3(blocks), RED_W * 32, 0, st, w->part, w->ranges, w->sums, w->ctas, weights, grad,
+               w->squares, stats);
+  launch_early(k_update_adam, dim3((weights + 2 + 255) / 256), 256, 0, st, w->in, blocks, w->squares, c12, stats, theta,
+               grad, first, second, pack, reinterpret_cast<bf16*>(w->w1t));
   return cudaGetLastError();
 }
 
