@@ -16,15 +16,14 @@
 // Nearest-waypoint searches are exact brute force over a candidate list: a
 // block of 16 x 16 cells keeps, in ascending index order, every waypoint
 // whose distance to the block's bounding box could make it the nearest of
-// some cell or put it inside the ball of one (bounds with a relative margin
-// of 1e-9, far above the rounding of the distances), so each cell scans a
-// few waypoints in the order the full scan would. Ties go to the lower
-// index, as the reference's arrays show.
+// some cell or put it inside the ball of one (bounds in 32 bits with a margin
+// above their rounding), so each cell scans a few waypoints in the order the
+// full scan would. Ties go to the lower index, as the reference's arrays show.
 //
-// The feature transform is the separable exact Euclidean method of Maurer,
-// Qi and Raghavan (2003): per column the nearest feature row (ties to the
-// lower row), then per row the lower envelope of those candidates (ties to
-// the lower column). The blur is the 13-tap correlation of sigma 1.5 with
+// The feature transform is the separable exact Euclidean one: per column the
+// nearest feature row (ties to the lower row), then per row the nearest of
+// those candidates (ties to the lower column), found by halving the row: the
+// nearest candidate's column is monotone along it. The blur is the 13-tap correlation of sigma 1.5 with
 // reflected edges, axis 0 then axis 1, each output summed as its centre tap
 // and then symmetric pairs from the outermost inward.
 #include <cuda_runtime.h>
@@ -66,52 +65,83 @@ struct CellArgs {
 
 __device__ __forceinline__ double cell_x(double x0, double cell, int ix) { return x0 + cell * (double)ix; }
 
+// A waypoint's place from the corner of a block's box, in 32 bits.
+__device__ __forceinline__ float2 place(const CellArgs& a, int w, double2 corner) {
+  return make_float2((float)(a.route[3 * w] - corner.x), (float)(a.route[3 * w + 1] - corner.y));
+}
+
+// A block's candidate waypoints: their indices, ascending, and places. `margin` is above twice what rounding can do to
+// a difference of two squared distances: what differs by more is ordered as in
+// 64 bits, also after the square root. Infinite or NaN where a place is out of
+// range, so that 64 bits decide.
+struct Candidates {
+  const int* w;
+  const float2* at;
+  int n;
+  double2 corner;
+  float margin;
+};
+
 // One cell's nearest waypoint (*nearest) and, for a ball query, its passes
-// and the nearest waypoint of each, over the candidates `cw` (indices,
-// ascending) with coordinates `cxy` (racer/track.py:73-86 and 89).
-__device__ int cell_passes(const CellArgs& a, const int* cw, const double2* cxy, int n, double x, double y,
-                           int* out, int* nearest) {
+// and the nearest waypoint of each (racer/track.py:73-86 and 89). (fx, fy) is
+// the cell's place from the corner of the block's box. Distances are compared
+// in 32 bits and again in 64 where those leave it open: 64-bit arithmetic runs
+// at 1/64 of the 32-bit rate, and comparing every candidate in it, with a
+// square root for each within the ball, took 257 us for 721 x 441 cells and
+// 285 waypoints against 55.
+template <bool ALL>
+__device__ int cell_passes(const CellArgs& a, const Candidates& cand, double x, double y, float fx, float fy, int* out,
+                           int* nearest) {
+  auto square = [&](int w) {
+    const double dx = a.route[3 * w] - x, dy = a.route[3 * w + 1] - y;
+    return dx * dx + dy * dy;
+  };
+  auto farther = [&](int u, int w) { return sqrt(square(w)) < sqrt(square(u)); };  // w is nearer than u
+  const bool ball = a.r2 >= 0.0;
+  const float r2 = (float)a.r2, margin = cand.margin;
   int pbest[MAX_PASSES];
-  double pd[MAX_PASSES];
-  int np = 0, first = -1, last = -10, best = 0;
-  double bd2 = INFINITY;
-  for (int i = 0; i < n; ++i) {
-    const int w = cw ? cw[i] : i;
-    const double2 r = cxy ? cxy[i] : make_double2(a.route[3 * w], a.route[3 * w + 1]);
-    const double dx = r.x - x, dy = r.y - y;
-    const double d2 = dx * dx + dy * dy;
-    if (d2 < bd2) bd2 = d2, best = w;
-    if (!(d2 <= a.r2)) continue;
-    const double d = sqrt(d2);
+  int np = 0, first = -1, last = -10, best = -1, pass = 0;  // pass: the nearest of the last one
+  float bd = INFINITY, pd = 0.0f;                           // squared
+  for (int i = 0; i < cand.n; ++i) {
+    const int w = ALL ? i : cand.w[i];
+    const float2 at = ALL ? place(a, w, cand.corner) : cand.at[i];
+    const float dx = at.x - fx, dy = at.y - fy, d2 = dx * dx + dy * dy;
+    if (d2 < bd - margin) {
+      bd = d2, best = w;
+    } else if (!(d2 > bd + margin)) {
+      const double q = square(w);
+      if (q < (best < 0 ? INFINITY : square(best))) bd = d2, best = w;
+    }
+    if (!ball || d2 > r2 + margin) continue;
+    if (!(d2 < r2 - margin) && !(square(w) <= a.r2)) continue;
     if (np == 0 || w - last > 2) {  // a gap of more than 2 starts a new pass
       if (np == MAX_PASSES) return -1;
-      pbest[np] = w, pd[np] = d, ++np;
-    } else if (d < pd[np - 1]) {
-      pbest[np - 1] = w, pd[np - 1] = d;
+      if (np) pbest[np - 1] = pass;
+      pass = w, pd = d2, ++np;
+    } else if (d2 < pd - margin || (!(d2 > pd + margin) && farther(pass, w))) {
+      pass = w, pd = d2;
     }
     if (first < 0) first = w;
     last = w;
   }
-  *nearest = best;
+  *nearest = best < 0 ? 0 : best;
   if (np == 0) return 0;
+  pbest[np - 1] = pass;
   if (np > 1 && first == 0 && last == a.W - 1) {  // the pass through the seam: its end, then its start
-    int bw = pbest[np - 1];
-    double bd = pd[np - 1];
-    if (pd[0] < bd) bw = pbest[0], bd = pd[0];
-    pbest[0] = bw, pd[0] = bd, --np;
+    if (farther(pbest[np - 1], pbest[0])) pbest[np - 1] = pbest[0];
+    pbest[0] = pbest[np - 1], --np;
   }
   for (int i = 1; i < np; ++i) {  // stable sort by height
     const int w = pbest[i];
-    const double d = pd[i], z = a.route[3 * w + 2];
+    const double z = a.route[3 * w + 2];
     int j = i;
-    while (j > 0 && a.route[3 * pbest[j - 1] + 2] > z) pbest[j] = pbest[j - 1], pd[j] = pd[j - 1], --j;
-    pbest[j] = w, pd[j] = d;
+    while (j > 0 && a.route[3 * pbest[j - 1] + 2] > z) pbest[j] = pbest[j - 1], --j;
+    pbest[j] = w;
   }
   if (a.route[3 * pbest[np - 1] + 2] - a.route[3 * pbest[0] + 2] < 0.3) {  // one level: the nearest pass
     int bw = pbest[0];
-    double bd = pd[0];
     for (int i = 1; i < np; ++i)
-      if (pd[i] < bd) bw = pbest[i], bd = pd[i];
+      if (farther(bw, pbest[i])) bw = pbest[i];
     out[0] = bw;
     return 1;
   }
@@ -120,9 +150,9 @@ __device__ int cell_passes(const CellArgs& a, const int* cw, const double2* cxy,
 }
 
 __global__ void __launch_bounds__(TILE * TILE) k_cells(CellArgs a) {
-  __shared__ double2 s_xy[CAND_MAX];
+  __shared__ float2 s_at[CAND_MAX];
   __shared__ int s_w[CAND_MAX];
-  __shared__ double s_min[TILE * TILE / 32];
+  __shared__ float s_min[TILE * TILE / 32];
   __shared__ int s_warp[TILE * TILE / 32];
   __shared__ int s_total;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -130,30 +160,37 @@ __global__ void __launch_bounds__(TILE * TILE) k_cells(CellArgs a) {
   const double bx0 = cell_x(a.x0, a.cell, ix0), bx1 = cell_x(a.x0, a.cell, min(ix0 + TILE - 1, a.nx - 1));
   const double by0 = cell_x(a.y0, a.cell, iy0), by1 = cell_x(a.y0, a.cell, min(iy0 + TILE - 1, a.ny - 1));
 
+  const double2 corner = make_double2(bx0, by0);
+  const float ex = (float)(bx1 - bx0), ey = (float)(by1 - by0);
+
   // the smallest, over waypoints, of the distance to the box's farthest point
-  double m = INFINITY;
+  float m = INFINITY;
   for (int w = tid; w < a.W; w += blockDim.x) {
-    const double rx = a.route[3 * w], ry = a.route[3 * w + 1];
-    const double fx = fmax(fabs(rx - bx0), fabs(rx - bx1)), fy = fmax(fabs(ry - by0), fabs(ry - by1));
-    m = fmin(m, fx * fx + fy * fy);
+    const float2 p = place(a, w, corner);
+    const float fx = fmaxf(fabsf(p.x), fabsf(p.x - ex)), fy = fmaxf(fabsf(p.y), fabsf(p.y - ey));
+    m = fminf(m, fx * fx + fy * fy);
   }
-  for (int o = 16; o; o >>= 1) m = fmin(m, __shfl_xor_sync(0xffffffffu, m, o));
+  for (int o = 16; o; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (lane == 0) s_min[warp] = m;
   if (tid == 0) s_total = 0;
   __syncthreads();
   m = s_min[0];
-  for (int i = 1; i < TILE * TILE / 32; ++i) m = fmin(m, s_min[i]);
-  const double thr = fmax(m, a.r2) * (1.0 + 1e-9) + 1e-9;
+  for (int i = 1; i < TILE * TILE / 32; ++i) m = fminf(m, s_min[i]);
+  // Places within sqrt(thr) of the box are at most `reach` long, which is off by 2^-24 of it; so are a cell's. A squared
+  // distance between the two is off by 20 x 2^-24 reach^2 at most.
+  float thr = fmaxf(m, (float)a.r2) * (1.0f + 1e-5f) + 1e-36f;
+  const float reach = sqrtf(thr) + fmaxf(ex, ey), margin = reach * reach * 0x1p-16f + 1e-36f;
+  thr += margin;
 
   // candidates: waypoints whose distance to the box is within thr, in index order
   bool overflow = false;
   for (int base = 0; base < a.W; base += blockDim.x) {
     const int w = base + tid;
     bool take = false;
-    double rx = 0.0, ry = 0.0;
+    float2 p = make_float2(0.0f, 0.0f);
     if (w < a.W) {
-      rx = a.route[3 * w], ry = a.route[3 * w + 1];
-      const double dx = fmax(fmax(bx0 - rx, rx - bx1), 0.0), dy = fmax(fmax(by0 - ry, ry - by1), 0.0);
+      p = place(a, w, corner);
+      const float dx = fmaxf(fmaxf(-p.x, p.x - ex), 0.0f), dy = fmaxf(fmaxf(-p.y, p.y - ey), 0.0f);
       take = dx * dx + dy * dy <= thr;
     }
     const unsigned ballot = __ballot_sync(0xffffffffu, take);
@@ -162,7 +199,7 @@ __global__ void __launch_bounds__(TILE * TILE) k_cells(CellArgs a) {
     int offset = s_total;
     for (int i = 0; i < warp; ++i) offset += s_warp[i];
     offset += __popc(ballot & ((1u << lane) - 1u));
-    if (take && offset < CAND_MAX) s_w[offset] = w, s_xy[offset] = make_double2(rx, ry);
+    if (take && offset < CAND_MAX) s_w[offset] = w, s_at[offset] = p;
     __syncthreads();
     if (tid == 0)
       for (int i = 0; i < TILE * TILE / 32; ++i) s_total += s_warp[i];
@@ -175,11 +212,11 @@ __global__ void __launch_bounds__(TILE * TILE) k_cells(CellArgs a) {
   if (ix >= a.nx || iy >= a.ny) return;
   const double x = cell_x(a.x0, a.cell, ix), y = cell_x(a.y0, a.cell, iy);
   const long k = (long)iy * a.nx + ix;
-  const int n = overflow ? a.W : total;
-  const int* cw = overflow ? nullptr : s_w;
-  const double2* cxy = overflow ? nullptr : s_xy;
+  const Candidates cand{s_w, s_at, overflow ? a.W : total, corner, margin};
   int out[MAX_PASSES], best = 0;
-  const int got = cell_passes(a, cw, cxy, n, x, y, out, &best);
+  const float fx = (float)(x - corner.x), fy = (float)(y - corner.y);
+  const int got = overflow ? cell_passes<true>(a, cand, x, y, fx, fy, out, &best)
+                           : cell_passes<false>(a, cand, x, y, fx, fy, out, &best);
   a.nearest[k] = best;
   if (a.r2 < 0.0) return;
   if (got < 0) {
@@ -308,63 +345,71 @@ __global__ void __launch_bounds__(FT_WARPS * 32) k_ft_columns(const unsigned cha
   }
 }
 
-__device__ void ft_row(const int* row, int y, int nx, int* gs, int* out) {
-  int l = -1;
-  for (int x = 0; x < nx; ++x) {
-    const int fx = row[x];
-    if (fx < 0) continue;
-    const long long wR = (long long)(fx - y) * (fx - y);
-    while (l >= 1) {
-      const int v = gs[l], u = gs[l - 1];
-      const long long a = v - u, b = x - v, c = a + b;
-      const long long vR = (long long)(row[v] - y) * (row[v] - y), uR = (long long)(row[u] - y) * (row[u] - y);
-      if (c * vR - b * uR - a * wR - a * b * c <= 0) break;
-      --l;
-    }
-    gs[++l] = x;
-  }
-  if (l < 0) {
-    for (int x = 0; x < nx; ++x) out[x] = -1;
-    return;
-  }
-  const int maxl = l;
-  l = 0;
-  for (int x = 0; x < nx; ++x) {
-    int gl = gs[l];
-    long long d1 = (long long)(gl - x) * (gl - x) + (long long)(row[gl] - y) * (row[gl] - y);
-    while (l < maxl) {
-      const int gn = gs[l + 1];
-      const long long d2 = (long long)(gn - x) * (gn - x) + (long long)(row[gn] - y) * (row[gn] - y);
-      if (d1 <= d2) break;
-      d1 = d2, ++l, gl = gn;
-    }
-    out[x] = row[gl] * nx + gl;
-  }
-}
-
-// Per row, the lower envelope of the columns' candidates and, for every cell,
-// the flat index of its nearest feature (-1 when the grid has none). The
-// envelope is sequential: one thread walks the row, in shared memory when
-// SHARED (a warp per row stages the row, its stack and its output there),
-// else in global memory (`g` holds the stacks).
-template <bool SHARED>
-__global__ void k_ft_rows(const int* fy, int ny, int nx, int* g, int* src) {
+// Per row, the flat index of every cell's nearest feature (-1 when the grid
+// has none); of equally near ones, the lowest column's. That column never
+// falls from one cell of a row to the next, so a cell halfway between two
+// solved ones searches only the columns from the one's answer to the other's:
+// a warp per cell down to every 32nd cell, then a lane per cell over the
+// columns that the 31 cells between share, nx (1 + log2(nx / 32) / 32) warp
+// steps a row at most. D holds a squared distance. A block per row; the row is
+// staged in shared memory when STAGED. Bound by the few steps in turn that the
+// last segments take: 441 rows of 721 cells take 17 us (a thread per row,
+// walking its lower envelope: 210 us).
+constexpr int FT_ROW_WARPS = 8;
+template <class D, bool STAGED>
+__global__ void __launch_bounds__(FT_ROW_WARPS * 32) k_ft_rows(const int* __restrict__ fy, int nx, int* src) {
   extern __shared__ int ft_smem[];
-  const int y = SHARED ? blockIdx.x : blockIdx.x * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
+  const int y = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int* row = fy + (long)y * nx;
-  int* gs = g + (long)y * nx;
-  int* out = src + (long)y * nx;
-  if (SHARED) {
-    for (int x = threadIdx.x; x < nx; x += 32) ft_smem[x] = row[x];
-    __syncwarp();
-    row = ft_smem, gs = ft_smem + nx, out = ft_smem + 2 * nx;
-    if (threadIdx.x == 0) ft_row(row, y, nx, gs, out);
-    __syncwarp();
-    for (int x = threadIdx.x; x < nx; x += 32) src[(long)y * nx + x] = out[x];
-    return;
+  int* out = src + (long)y * nx;  // solved cells are read back by the other warps of the block
+  if (STAGED) {
+    for (int x = threadIdx.x; x < nx; x += FT_ROW_WARPS * 32) ft_smem[x] = row[x];
+    __syncthreads();
+    row = ft_smem;
   }
-  ft_row(row, y, nx, gs, out);
+  constexpr D FAR = sizeof(D) == 4 ? (D)INT_MAX : (D)LLONG_MAX;
+  auto distance = [&](int f, int column, int x) {
+    const D dy = f - y, dx = column - x;
+    return f < 0 ? FAR : dx * dx + dy * dy;
+  };
+  auto column_of = [&](int x, int none) { return x < 0 || x >= nx || out[x] < 0 ? none : out[x] % nx; };
+  int top = 32;
+  while (top < nx) top *= 2;
+  for (int step = top; step >= 32; step >>= 1) {  // cells 0, then the odd multiples of each step
+    for (long i = warp;; i += FT_ROW_WARPS) {
+      const long at = step == top ? i * step : (2 * i + 1) * step;
+      if (at >= nx) break;
+      const int x = (int)at;
+      const int lo = step == top ? 0 : column_of(x - step, 0);
+      const int hi = step == top ? nx - 1 : column_of(at + step < nx ? x + step : -1, nx - 1);
+      D best = FAR;
+      int column = -1;
+      for (int c = lo + lane; c <= hi; c += 32) {
+        const D d = distance(row[c], c, x);
+        if (d < best) best = d, column = c;
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        const D d = __shfl_xor_sync(0xffffffffu, best, o);
+        const int c = __shfl_xor_sync(0xffffffffu, column, o);
+        if (d < best || (d == best && (unsigned)c < (unsigned)column)) best = d, column = c;
+      }
+      if (lane == 0) out[x] = column < 0 ? -1 : row[column] * nx + column;
+    }
+    __syncthreads();
+  }
+  for (int x0 = warp * 32; x0 < nx; x0 += FT_ROW_WARPS * 32) {
+    const int lo = column_of(x0, 0), hi = column_of(nx - x0 > 32 ? x0 + 32 : -1, nx - 1);
+    const int x = min(x0 + lane, nx - 1);
+    D best = FAR;
+    int column = -1;
+#pragma unroll 4
+    for (int c = lo; c <= hi; ++c) {
+      const D d = distance(row[c], c, x);
+      if (d < best) best = d, column = c;
+    }
+    if (lane && x0 + lane < nx) out[x] = column < 0 ? -1 : row[column] * nx + column;
+  }
 }
 
 __global__ void k_gather(const double* height, const int* src, long cells, double* filled) {
@@ -452,18 +497,22 @@ struct Scratch {
 inline unsigned blocks(long n, int t) { return (unsigned)((n + t - 1) / t); }
 
 // The feature transform of `feature` into `src` (flat index of each cell's
-// nearest feature); fy and g are [cells] scratch.
-cudaError_t feature_transform(const unsigned char* feature, int ny, int nx, int* fy, int* g, int* src, cudaStream_t st) {
+// nearest feature); fy is [cells] scratch.
+template <class D>
+void feature_rows(const int* fy, int ny, int nx, int* src, cudaStream_t st) {
+  const size_t smem = sizeof(int) * (size_t)nx;
+  if (smem <= 48 * 1024)
+    k_ft_rows<D, true><<<ny, FT_ROW_WARPS * 32, smem, st>>>(fy, nx, src);
+  else
+    k_ft_rows<D, false><<<ny, FT_ROW_WARPS * 32, 0, st>>>(fy, nx, src);
+}
+
+cudaError_t feature_transform(const unsigned char* feature, int ny, int nx, int* fy, int* src, cudaStream_t st) {
   k_ft_columns<<<blocks(nx, FT_WARPS), FT_WARPS * 32, 0, st>>>(feature, ny, nx, fy);
-  const size_t smem = 3 * sizeof(int) * (size_t)nx;
-  if (smem <= 48 * 1024 ||
-      (smem <= 200 * 1024 &&
-       cudaFuncSetAttribute(k_ft_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)) {
-    k_ft_rows<true><<<ny, 32, smem, st>>>(fy, ny, nx, g, src);
-  } else {
-    cudaGetLastError();
-    k_ft_rows<false><<<blocks(ny, 64), 64, 0, st>>>(fy, ny, nx, g, src);
-  }
+  if ((nx > ny ? nx : ny) <= 32767)  // a squared distance fits 32 bits
+    feature_rows<int>(fy, ny, nx, src, st);
+  else
+    feature_rows<long long>(fy, ny, nx, src, st);
   return cudaGetLastError();
 }
 
@@ -487,18 +536,17 @@ int pack(Scratch& s, int layers, double* clearance, double* height, const int* w
     TRACK_LAUNCH();
   }
   unsigned char* feature;
-  int *fy, *g, *src;
+  int *fy, *src;
   double *filled, *tmp;
   RACER_TRY(s.get(&feature, cells));
   RACER_TRY(s.get(&fy, cells));
-  RACER_TRY(s.get(&g, cells));
   RACER_TRY(s.get(&src, cells));
   RACER_TRY(s.get(&filled, cells));
   RACER_TRY(s.get(&tmp, cells));
   const Blur b = blur_weights();
   for (int l = 0; l < layers; ++l) {
     k_mask_road<<<blocks(cells, T), T, 0, st>>>(clearance + l * cells, cells, feature);
-    RACER_TRY(feature_transform(feature, ny, nx, fy, g, src, st));
+    RACER_TRY(feature_transform(feature, ny, nx, fy, src, st));
     TRACK_LAUNCH();
     int first = 0;
     RACER_TRY(cudaMemcpyAsync(&first, src, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -644,7 +692,7 @@ int racer_track_image(const uint8_t* free_, const double* route, int W, double x
   Scratch s;
   double *d_route, *clearance, *height;
   unsigned char *d_free, *wall, *open;
-  int *nearest, *to_wall, *to_open, *fy, *g, *flags;
+  int *nearest, *to_wall, *to_open, *fy, *flags;
   float* d_grids;
   RampRow* d_ramps = nullptr;
   RACER_TRY(s.get(&d_route, 3 * (size_t)W));
@@ -655,7 +703,6 @@ int racer_track_image(const uint8_t* free_, const double* route, int W, double x
   RACER_TRY(s.get(&to_wall, cells));
   RACER_TRY(s.get(&to_open, cells));
   RACER_TRY(s.get(&fy, cells));
-  RACER_TRY(s.get(&g, cells));
   RACER_TRY(s.get(&flags, 2));
   RACER_TRY(s.get(&clearance, cells));
   RACER_TRY(s.get(&height, cells));
@@ -672,8 +719,8 @@ int racer_track_image(const uint8_t* free_, const double* route, int W, double x
   k_cells<<<dim3(blocks(nx, TILE), blocks(ny, TILE)), TILE * TILE, 0, st.s>>>(ca);
   k_mask_image<<<blocks(cells, 256), 256, 0, st.s>>>(d_free, cells, wall, open);
   TRACK_LAUNCH();
-  RACER_TRY(feature_transform(wall, ny, nx, fy, g, to_wall, st.s));
-  RACER_TRY(feature_transform(open, ny, nx, fy, g, to_open, st.s));
+  RACER_TRY(feature_transform(wall, ny, nx, fy, to_wall, st.s));
+  RACER_TRY(feature_transform(open, ny, nx, fy, to_open, st.s));
   int first[2] = {0, 0};
   RACER_TRY(cudaMemcpyAsync(&first[0], to_wall, sizeof(int), cudaMemcpyDeviceToHost, st.s));
   RACER_TRY(cudaMemcpyAsync(&first[1], to_open, sizeof(int), cudaMemcpyDeviceToHost, st.s));
