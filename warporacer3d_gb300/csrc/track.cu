@@ -306,42 +306,40 @@ __global__ void k_mask_image(const unsigned char* free_, long cells, unsigned ch
   if (k < cells) wall[k] = free_[k] == 0, open[k] = free_[k] != 0;
 }
 
-// Per column, the nearest feature row (ties to the lower row), -1 if none: one
-// warp per column, the last feature at or above each row as a running
-// maximum over chunks of 32 rows, then the first at or below as a running
-// minimum from the bottom.
-constexpr int FT_WARPS = 8;
-__global__ void __launch_bounds__(FT_WARPS * 32) k_ft_columns(const unsigned char* feature, int ny, int nx, int* fy) {
-  const int x = blockIdx.x * FT_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (x >= nx) return;  // warp-uniform
-  int carry = -1;
-  for (int y0 = 0; y0 < ny; y0 += 32) {
-    const int y = y0 + lane;
-    int p = (y < ny && feature[(long)y * nx + x]) ? y : -1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int q = __shfl_up_sync(0xffffffffu, p, o);
-      if (lane >= o) p = max(p, q);
-    }
-    p = max(p, carry);
-    if (y < ny) fy[(long)y * nx + x] = p;
-    carry = __shfl_sync(0xffffffffu, p, 31);
+// Per column, the nearest feature row (ties to the lower row), -1 if none: a
+// block per 32 columns, a lane each, a warp per stretch of the rows. Each warp
+// finds the first and last feature of its stretch, from which every stretch
+// gets the last one above it and the first below; then it walks its rows down
+// and up. Rows of 32 cells are read and written together (a warp per column,
+// its lanes down the rows, took 22.5 us for 721 x 441 cells; this takes 11.2).
+constexpr int FT_WARPS = 32;
+__global__ void __launch_bounds__(FT_WARPS * 32) k_ft_columns(const unsigned char* __restrict__ feature, int ny, int nx,
+                                                              int* fy) {
+  __shared__ int s_first[FT_WARPS][32], s_last[FT_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, x = blockIdx.x * 32 + lane;
+  const int rows = (ny + FT_WARPS - 1) / FT_WARPS, y0 = min(warp * rows, ny), y1 = min(y0 + rows, ny);
+  int first = INT_MAX, last = -1;
+  if (x < nx) {
+#pragma unroll 8
+    for (int y = y0; y < y1; ++y)
+      if (feature[(long)y * nx + x]) first = min(first, y), last = y;
   }
-  int below = INT_MAX;
-  for (int y0 = ((ny - 1) / 32) * 32; y0 >= 0; y0 -= 32) {
-    const int y = y0 + lane;
-    int q = (y < ny && feature[(long)y * nx + x]) ? y : INT_MAX;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int r = __shfl_down_sync(0xffffffffu, q, o);
-      if (lane + o < 32) q = min(q, r);
-    }
-    q = min(q, below);
-    if (y < ny && q != INT_MAX) {
-      const int p = fy[(long)y * nx + x];
-      if (p < 0 || q - y < y - p) fy[(long)y * nx + x] = q;
-    }
-    below = __shfl_sync(0xffffffffu, q, 0);
+  s_first[warp][lane] = first, s_last[warp][lane] = last;
+  __syncthreads();
+  int above = -1, below = INT_MAX;
+  for (int i = 0; i < warp; ++i) above = max(above, s_last[i][lane]);
+  for (int i = warp + 1; i < FT_WARPS; ++i) below = min(below, s_first[i][lane]);
+  if (x >= nx) return;
+#pragma unroll 8
+  for (int y = y0; y < y1; ++y) {
+    if (feature[(long)y * nx + x]) above = y;
+    fy[(long)y * nx + x] = above;
+  }
+#pragma unroll 8
+  for (int y = y1 - 1; y >= y0; --y) {
+    const int p = fy[(long)y * nx + x];
+    if (p == y) below = y;
+    if (below != INT_MAX && (p < 0 || below - y < y - p)) fy[(long)y * nx + x] = below;
   }
 }
 
@@ -508,7 +506,7 @@ void feature_rows(const int* fy, int ny, int nx, int* src, cudaStream_t st) {
 }
 
 cudaError_t feature_transform(const unsigned char* feature, int ny, int nx, int* fy, int* src, cudaStream_t st) {
-  k_ft_columns<<<blocks(nx, FT_WARPS), FT_WARPS * 32, 0, st>>>(feature, ny, nx, fy);
+  k_ft_columns<<<blocks(nx, 32), FT_WARPS * 32, 0, st>>>(feature, ny, nx, fy);
   if ((nx > ny ? nx : ny) <= 32767)  // a squared distance fits 32 bits
     feature_rows<int>(fy, ny, nx, src, st);
   else
