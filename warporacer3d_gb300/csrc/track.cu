@@ -478,17 +478,46 @@ Blur blur_weights() {  // sigma 1.5, radius 6
   return b;
 }
 
-// Device buffers of one compilation, freed on every exit path.
+// Device buffers of one compilation, freed on every exit path: `get` names the
+// ones that `take` then lays out in one allocation (an allocation and its
+// release cost 20 us or more of host time each, and a ribbon has 19 buffers).
 struct Scratch {
+  struct Buffer {
+    void** p;
+    size_t bytes;
+  };
+  std::vector<Buffer> wanted;
   std::vector<void*> ptrs;
   ~Scratch() {
     for (void* p : ptrs) cudaFree(p);
   }
   template <class T>
-  cudaError_t get(T** p, size_t count) {
-    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T) + 16);
-    if (e == cudaSuccess) ptrs.push_back(*p);
-    return e;
+  void get(T** p, size_t count) {
+    wanted.push_back({(void**)p, (count * sizeof(T) + 255) / 256 * 256});
+  }
+  cudaError_t take() {
+    size_t total = 0;
+    for (const Buffer& b : wanted) total += b.bytes;
+    char* at = nullptr;
+    if (cudaError_t e = cudaMalloc((void**)&at, total); e != cudaSuccess) return e;
+    ptrs.push_back(at);
+    for (const Buffer& b : wanted) *b.p = at, at += b.bytes;
+    wanted.clear();
+    return cudaSuccess;
+  }
+};
+
+// What `pack` needs besides its grids.
+struct PackScratch {
+  unsigned char* feature;
+  int *fy, *src;
+  double *filled, *tmp;
+  void get(Scratch& s, size_t cells) {
+    s.get(&feature, cells);
+    s.get(&fy, cells);
+    s.get(&src, cells);
+    s.get(&filled, cells);
+    s.get(&tmp, cells);
   }
 };
 
@@ -525,7 +554,7 @@ cudaError_t feature_transform(const unsigned char* feature, int ny, int nx, int*
 
 // racer/track.py:108-125 from the device grids: ramps, off-road fill, blur,
 // float32 grids [layers][3][cells] into `grids` (device).
-int pack(Scratch& s, int layers, double* clearance, double* height, const int* waypoint, const RampRow* ramps_dev,
+int pack(const PackScratch& s, int layers, double* clearance, double* height, const int* waypoint, const RampRow* ramps_dev,
          int n_ramps, double x0, double y0, double cell, int nx, int ny, float* grids, cudaStream_t st) {
   const long cells = (long)nx * ny;
   const int T = 256;
@@ -533,30 +562,22 @@ int pack(Scratch& s, int layers, double* clearance, double* height, const int* w
     k_ramps<<<blocks(cells, T), T, 0, st>>>(ramps_dev, n_ramps, x0, y0, cell, nx, cells, layers, height);
     TRACK_LAUNCH();
   }
-  unsigned char* feature;
-  int *fy, *src;
-  double *filled, *tmp;
-  RACER_TRY(s.get(&feature, cells));
-  RACER_TRY(s.get(&fy, cells));
-  RACER_TRY(s.get(&src, cells));
-  RACER_TRY(s.get(&filled, cells));
-  RACER_TRY(s.get(&tmp, cells));
   const Blur b = blur_weights();
   for (int l = 0; l < layers; ++l) {
-    k_mask_road<<<blocks(cells, T), T, 0, st>>>(clearance + l * cells, cells, feature);
-    RACER_TRY(feature_transform(feature, ny, nx, fy, src, st));
+    k_mask_road<<<blocks(cells, T), T, 0, st>>>(clearance + l * cells, cells, s.feature);
+    RACER_TRY(feature_transform(s.feature, ny, nx, s.fy, s.src, st));
     TRACK_LAUNCH();
     int first = 0;
-    RACER_TRY(cudaMemcpyAsync(&first, src, sizeof(int), cudaMemcpyDeviceToHost, st));
+    RACER_TRY(cudaMemcpyAsync(&first, s.src, sizeof(int), cudaMemcpyDeviceToHost, st));
     RACER_TRY(cudaStreamSynchronize(st));
     if (first < 0) {
       racer_host::set_error("track: a layer has no road cell (clearance > 0)");
       return 3;
     }
     float* out = grids + (long)l * 3 * cells;
-    k_gather<<<blocks(cells, T), T, 0, st>>>(height + l * cells, src, cells, filled);
-    k_blur_rows<<<blocks(cells, T), T, 0, st>>>(filled, ny, nx, b, tmp);
-    k_blur_cols<<<blocks(cells, T), T, 0, st>>>(tmp, ny, nx, b, out + cells);
+    k_gather<<<blocks(cells, T), T, 0, st>>>(height + l * cells, s.src, cells, s.filled);
+    k_blur_rows<<<blocks(cells, T), T, 0, st>>>(s.filled, ny, nx, b, s.tmp);
+    k_blur_cols<<<blocks(cells, T), T, 0, st>>>(s.tmp, ny, nx, b, out + cells);
     k_write_layer<<<blocks(cells, T), T, 0, st>>>(clearance + l * cells, waypoint + l * cells, cells, out);
     TRACK_LAUNCH();
   }
@@ -595,15 +616,18 @@ int racer_track_ribbon(const double* route, const double* cos_h, const double* s
   double *d_route, *d_cos, *d_sin, *d_grade;
   int *nearest, *count, *pw, *flags;
   unsigned char* upper;
-  RACER_TRY(s.get(&d_route, 3 * (size_t)W));
-  RACER_TRY(s.get(&d_cos, W));
-  RACER_TRY(s.get(&d_sin, W));
-  RACER_TRY(s.get(&d_grade, W));
-  RACER_TRY(s.get(&nearest, cells));
-  RACER_TRY(s.get(&count, cells));
-  RACER_TRY(s.get(&pw, cells * MAX_PASSES));
-  RACER_TRY(s.get(&flags, 2));
-  RACER_TRY(s.get(&upper, W));
+  s.get(&d_route, 3 * (size_t)W);
+  s.get(&d_cos, W);
+  s.get(&d_sin, W);
+  s.get(&d_grade, W);
+  s.get(&nearest, cells);
+  s.get(&count, cells);
+  s.get(&pw, cells * MAX_PASSES);
+  s.get(&flags, 2);
+  s.get(&upper, W);
+  PackScratch ps;
+  ps.get(s, cells);
+  RACER_TRY(s.take());
   RACER_TRY(cudaMemcpyAsync(d_route, route, 3 * sizeof(double) * W, cudaMemcpyHostToDevice, st.s));
   RACER_TRY(cudaMemcpyAsync(d_cos, cos_h, sizeof(double) * W, cudaMemcpyHostToDevice, st.s));
   RACER_TRY(cudaMemcpyAsync(d_sin, sin_h, sizeof(double) * W, cudaMemcpyHostToDevice, st.s));
@@ -653,19 +677,19 @@ int racer_track_ribbon(const double* route, const double* cos_h, const double* s
   int* waypoint;
   float* d_grids;
   RampRow* d_ramps = nullptr;
-  RACER_TRY(s.get(&clearance, layers * cells));
-  RACER_TRY(s.get(&height, layers * cells));
-  RACER_TRY(s.get(&waypoint, layers * cells));
-  RACER_TRY(s.get(&d_grids, 3 * layers * cells));
-  if (n_ramps) {
-    RACER_TRY(s.get(&d_ramps, n_ramps));
+  s.get(&clearance, layers * cells);
+  s.get(&height, layers * cells);
+  s.get(&waypoint, layers * cells);
+  s.get(&d_grids, 3 * layers * cells);
+  if (n_ramps) s.get(&d_ramps, n_ramps);
+  RACER_TRY(s.take());
+  if (n_ramps)
     RACER_TRY(cudaMemcpyAsync(d_ramps, ramps, sizeof(RampRow) * n_ramps, cudaMemcpyHostToDevice, st.s));
-  }
   FillArgs fa{d_route, d_cos, d_sin, d_grade, nearest, count, pw, upper, half_width, bank, x0, y0, cell,
               nx, layers, 0, (f & 1) ? 1 : 0, cells, clearance, height, waypoint};
   k_fill<<<blocks(cells, 256), 256, 0, st.s>>>(fa);
   TRACK_LAUNCH();
-  int rc = pack(s, layers, clearance, height, waypoint, d_ramps, n_ramps, x0, y0, cell, nx, ny, d_grids, st.s);
+  int rc = pack(ps, layers, clearance, height, waypoint, d_ramps, n_ramps, x0, y0, cell, nx, ny, d_grids, st.s);
   if (rc) return rc;
   RACER_TRY(cudaMemcpyAsync(grids, d_grids, sizeof(float) * 3 * layers * cells, cudaMemcpyDeviceToHost, st.s));
   RACER_TRY(cudaStreamSynchronize(st.s));
@@ -690,35 +714,36 @@ int racer_track_image(const uint8_t* free_, const double* route, int W, double x
   Scratch s;
   double *d_route, *clearance, *height;
   unsigned char *d_free, *wall, *open;
-  int *nearest, *to_wall, *to_open, *fy, *flags;
+  int *nearest, *to_wall, *to_open, *flags;
   float* d_grids;
   RampRow* d_ramps = nullptr;
-  RACER_TRY(s.get(&d_route, 3 * (size_t)W));
-  RACER_TRY(s.get(&d_free, cells));
-  RACER_TRY(s.get(&wall, cells));
-  RACER_TRY(s.get(&open, cells));
-  RACER_TRY(s.get(&nearest, cells));
-  RACER_TRY(s.get(&to_wall, cells));
-  RACER_TRY(s.get(&to_open, cells));
-  RACER_TRY(s.get(&fy, cells));
-  RACER_TRY(s.get(&flags, 2));
-  RACER_TRY(s.get(&clearance, cells));
-  RACER_TRY(s.get(&height, cells));
-  RACER_TRY(s.get(&d_grids, 3 * cells));
+  s.get(&d_route, 3 * (size_t)W);
+  s.get(&d_free, cells);
+  s.get(&wall, cells);
+  s.get(&open, cells);
+  s.get(&nearest, cells);
+  s.get(&to_wall, cells);
+  s.get(&to_open, cells);
+  s.get(&flags, 2);
+  s.get(&clearance, cells);
+  s.get(&height, cells);
+  s.get(&d_grids, 3 * cells);
+  if (n_ramps) s.get(&d_ramps, n_ramps);
+  PackScratch ps;
+  ps.get(s, cells);
+  RACER_TRY(s.take());
   RACER_TRY(cudaMemcpyAsync(d_route, route, 3 * sizeof(double) * W, cudaMemcpyHostToDevice, st.s));
   RACER_TRY(cudaMemcpyAsync(d_free, free_, cells, cudaMemcpyHostToDevice, st.s));
   RACER_TRY(cudaMemsetAsync(flags, 0, 2 * sizeof(int), st.s));
   RACER_TRY(cudaMemsetAsync(height, 0, sizeof(double) * cells, st.s));
-  if (n_ramps) {
-    RACER_TRY(s.get(&d_ramps, n_ramps));
+  if (n_ramps)
     RACER_TRY(cudaMemcpyAsync(d_ramps, ramps, sizeof(RampRow) * n_ramps, cudaMemcpyHostToDevice, st.s));
-  }
   CellArgs ca{d_route, W, x0, y0, cell, nx, ny, -1.0, nearest, nullptr, nullptr, nullptr, flags + 1};
   k_cells<<<dim3(blocks(nx, TILE), blocks(ny, TILE)), TILE * TILE, 0, st.s>>>(ca);
   k_mask_image<<<blocks(cells, 256), 256, 0, st.s>>>(d_free, cells, wall, open);
   TRACK_LAUNCH();
-  RACER_TRY(feature_transform(wall, ny, nx, fy, to_wall, st.s));
-  RACER_TRY(feature_transform(open, ny, nx, fy, to_open, st.s));
+  RACER_TRY(feature_transform(wall, ny, nx, ps.fy, to_wall, st.s));
+  RACER_TRY(feature_transform(open, ny, nx, ps.fy, to_open, st.s));
   int first[2] = {0, 0};
   RACER_TRY(cudaMemcpyAsync(&first[0], to_wall, sizeof(int), cudaMemcpyDeviceToHost, st.s));
   RACER_TRY(cudaMemcpyAsync(&first[1], to_open, sizeof(int), cudaMemcpyDeviceToHost, st.s));
@@ -729,7 +754,7 @@ int racer_track_image(const uint8_t* free_, const double* route, int W, double x
   }
   k_image_clear<<<blocks(cells, 256), 256, 0, st.s>>>(d_free, to_wall, to_open, nx, cells, cell, clearance);
   TRACK_LAUNCH();
-  int rc = pack(s, 1, clearance, height, nearest, d_ramps, n_ramps, x0, y0, cell, nx, ny, d_grids, st.s);
+  int rc = pack(ps, 1, clearance, height, nearest, d_ramps, n_ramps, x0, y0, cell, nx, ny, d_grids, st.s);
   if (rc) return rc;
   RACER_TRY(cudaMemcpyAsync(grids, d_grids, sizeof(float) * 3 * cells, cudaMemcpyDeviceToHost, st.s));
   RACER_TRY(cudaStreamSynchronize(st.s));

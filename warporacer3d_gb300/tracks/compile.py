@@ -81,23 +81,42 @@ class ImageInput:
         return 3 * self.nx * self.ny
 
 
+HEADER = 12  # floats before the grids
+
+
+def _ends(inp, layers):
+    """The packed array's header and route (racer/track.py:122-125)."""
+    route, along = inp.route, arc(inp.route)
+    header = [inp.nx, inp.ny, inp.x0, inp.y0, inp.cell, len(route), along[-1] / len(route), layers, inp.slope, 0, 0, 0]
+    return (np.array(header, dtype=np.float64).astype(np.float32),
+            np.column_stack([route, headings(route)]).ravel().astype(np.float32))
+
+
 def assemble(inp, grids, layers):
     """Header, grids and route into the packed float32 array (racer/track.py:122-125)."""
-    route = inp.route
-    header = [inp.nx, inp.ny, inp.x0, inp.y0, inp.cell, len(route), arc(route)[-1] / len(route), layers, inp.slope,
-              0, 0, 0]
-    head = np.array(header, dtype=np.float64).astype(np.float32)
-    tail = np.column_stack([route, headings(route)]).ravel().astype(np.float32)
+    head, tail = _ends(inp, layers)
     return np.concatenate([head, grids[:layers * 3 * inp.nx * inp.ny], tail])
+
+
+def _compile(inp, run, what):
+    """The packed array of `inp`, its grids written in place by the C ABI's `what` through `run`."""
+    out = np.empty(HEADER + inp.grids_len() + 4 * len(inp.route), dtype=np.float32)
+    rc, _, layers = run(inp, getattr(_lib(), what), out[HEADER:HEADER + inp.grids_len()])
+    _check(rc, what)
+    head, tail = _ends(inp, layers)
+    end = HEADER + layers * 3 * inp.nx * inp.ny
+    out[:HEADER], out[end:end + tail.size] = head, tail
+    out.resize(end + tail.size, refcheck=False)  # a one-layer ribbon's array ends early; no view of it is left
+    return out
 
 
 def _dp(a):
     return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
 
 
-def ribbon_grids(inp, fn):
-    """Run a ribbon grid compiler `fn` (the C ABI's signature) on `inp`: (grids, layers)."""
-    grids = np.empty(inp.grids_len(), dtype=np.float32)
+def ribbon_grids(inp, fn, grids=None):
+    """Run a ribbon grid compiler `fn` (the C ABI's signature) on `inp`, into `grids` if given: (rc, grids, layers)."""
+    grids = np.empty(inp.grids_len(), dtype=np.float32) if grids is None else grids
     layers = ctypes.c_int(0)
     ramps = np.ascontiguousarray(inp.ramps)
     rc = fn(_dp(inp.route), _dp(inp.cos_h), _dp(inp.sin_h), _dp(inp.grade), len(inp.route),
@@ -107,9 +126,9 @@ def ribbon_grids(inp, fn):
     return rc, grids, layers.value
 
 
-def image_grids(inp, fn):
-    """Run an image grid compiler `fn` on `inp`: (grids, 1)."""
-    grids = np.empty(inp.grids_len(), dtype=np.float32)
+def image_grids(inp, fn, grids=None):
+    """Run an image grid compiler `fn` on `inp`, into `grids` if given: (rc, grids, 1)."""
+    grids = np.empty(inp.grids_len(), dtype=np.float32) if grids is None else grids
     ramps = np.ascontiguousarray(inp.ramps)
     rc = fn(inp.free.ctypes.data_as(ctypes.POINTER(ctypes.c_uint8)), _dp(inp.route), len(inp.route),
             float(inp.x0), float(inp.y0), float(inp.cell), inp.nx, inp.ny, _dp(ramps), len(ramps),
@@ -131,19 +150,13 @@ def _check(rc, what):
 def ribbon(route, half_width, bank, cell, ramps=()):
     """A road `half_width` either side of `route` rising `bank` per metre outward,
     compiled on the GPU (racer/track.py:61-125)."""
-    inp = RibbonInput(route, half_width, bank, cell, ramps)
-    rc, grids, layers = ribbon_grids(inp, _lib().racer_track_ribbon)
-    _check(rc, "racer_track_ribbon")
-    return assemble(inp, grids, layers)
+    return _compile(RibbonInput(route, half_width, bank, cell, ramps), ribbon_grids, "racer_track_ribbon")
 
 
 def compile_image(free, loop, x0, y0, cell, ramps=()):
     """Free-space image (rows south to north) + centreline loop (row, col) -> packed
     one-layer track, compiled on the GPU (racer/track.py:54-58, 108-125)."""
-    inp = ImageInput(free, loop, x0, y0, cell, ramps)
-    rc, grids, layers = image_grids(inp, _lib().racer_track_image)
-    _check(rc, "racer_track_image")
-    return assemble(inp, grids, layers)
+    return _compile(ImageInput(free, loop, x0, y0, cell, ramps), image_grids, "racer_track_image")
 
 
 def builtin_route(name):
