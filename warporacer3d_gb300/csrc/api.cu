@@ -221,6 +221,8 @@ static int upload_track(const float* track, size_t len, float** d_track, float2*
         lc[q] = slot(d0 || !d1 ? v0 : v1);
         lc[q + 1] = d0 && d1 ? slot(v1) : make_float2(off, nan);
       }
+    if (L == 2)  // both clearances, then both heights, which the march subtracts as a pair
+      for (size_t k = 0; k < lidar; k += 2) std::swap(lc[k].y, lc[k + 1].x);
   }
   if (int rc = dalloc(d_track, len)) return rc;
   if (int rc = dalloc(d_cl, cl.size())) return rc;

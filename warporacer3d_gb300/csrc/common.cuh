@@ -46,8 +46,8 @@ struct TrackDev {
   float band;      // 0.5 - (5.001 max(nx, ny) + 4.001 max(|x0|, |y0|) / cell + 16) 2^-24: no division inside +-band
   float nxf, nyf;
   long route;
-  // The lidar's cells for one or two layers (sim.cu, lidar_probe): float2 or
-  // float4 per cell, rows of lw = nx + 1 cells over ny + 1 rows, the last
+  // The lidar's cells for one or two layers (sim.cu, lidar_probe): float2
+  // (clearance, height) or float4 (both clearances, both heights) per cell, rows of lw = nx + 1 cells over ny + 1 rows, the last
   // column and row off-map cells; null for three or more layers.
   const float* lc;
   int lw;
