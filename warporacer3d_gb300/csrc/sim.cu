@@ -1012,22 +1012,19 @@ static LidarGrid lidar_grid(const Segments& g, const LidarShape& shape) {
 // SM keeps the split of the last kernel that needed more (a policy forward or a
 // learned lidar of another stream) until it drains, which under a long lidar it
 // does not: with 28 KB of L1 the step of 119,808 cars on five tracks takes
-// 7.2 ms, with this 6.1. The switch waits for the SM to drain, so small grids do
+// 7.2 ms, with this 6.1 (before the march's later gains). The switch waits for the SM to drain, so small grids do
 // without (4352 blocks, one of 16 rollout chains: 6.45 ms a rollout against 6.88).
 constexpr long BIG_LIDAR = 1 << 18;
 template <class... P, class... A>
 static void lidar_launch(void (*k)(P...), dim3 grid, unsigned threads, cudaStream_t st, bool early, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.stream = st;
-  cudaLaunchAttribute at{};
-  if ((long)grid.x * grid.y >= BIG_LIDAR) {
-    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    at.val.sharedMemCarveout = 14;  // per cent of 228 KB
-  } else {
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = early;
-  }
-  cfg.attrs = &at, cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = early;
+  at[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+  at[1].val.sharedMemCarveout = 14;  // per cent of 228 KB
+  cfg.attrs = at, cfg.numAttrs = (long)grid.x * grid.y >= BIG_LIDAR ? 2 : 1;
   cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
@@ -1096,6 +1093,17 @@ static void lidar_shape(const Segments& g, const LidarShape& shape, const float4
   }
   const LidarGrid lg = lidar_grid(g, shape);
   dim3 grid(lg.block0[g.count], (beams + 31) / 32);
+  // A launch a segment once there is work enough to hide their tails: the segment table leaves the march too few of its
+  // 32 registers and reads the track through an index. 16,000 cars x 1081 beams on five tracks (272,000 blocks) take
+  // 731 us a step against 835 and 119,808 cars 5.12 ms against 5.77, but 8000 cars (136,000 blocks, alone) 519 us
+  // against 502 and 2000 cars of 540 beams 93 us against 69.
+  if ((long)grid.x * grid.y >= BIG_LIDAR) {
+    LidarShape one = shape;
+    one.dynamic = 0;  // as the table's
+    for (int j = 0; j < g.count; ++j)
+      lidar_segment<CARS, WIDE>(g, lg.order[j], ray, obs, n, beams, beam_dir, iters, st, one, true);
+    return;
+  }
   lidar_launch(k_lidar_segments<CARS, WIDE>, grid, CARS * 32, st, true, g, lg, ray, obs, n, beams, beam_dir, iters);
 }
 
