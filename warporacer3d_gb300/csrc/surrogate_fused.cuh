@@ -69,9 +69,9 @@ __device__ __forceinline__ float world_store16(const float* v, const float* bias
     const __half2 t = __floats2half2_rn(y[2 * j], y[2 * j + 1]);
     w[j] = *reinterpret_cast<const uint32_t*>(&t);
   }
-  uint4* dst = reinterpret_cast<uint4*>(row + o0);
-  dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(__cvta_generic_to_global(row + o0)),
+               "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
   float mn = 1.0f;
   if (b0 + 15 < beams) {  // wholly inside
 #pragma unroll
@@ -130,43 +130,52 @@ __device__ __forceinline__ bool sf_wait(uint64_t* bar, uint32_t parity, volatile
 __device__ bool sf_producer(const CUtensorMap* tx, const CUtensorMap* tw1, const CUtensorMap* tw2,
                             const CUtensorMap* tw3, const CUtensorMap* tw4, uint8_t* abuf, uint8_t* stages,
                             const SfBars& b, int tiles, int nc, uint32_t* issued, uint32_t* xloads) {
-  uint32_t it = 0, local = 0;
+  uint32_t s = 0, parity = 1, local = 0;  // a stage's first use waits for nothing
+  auto stage = [&](const CUtensorMap* map, int kb, int row) {
+    if (*issued >= (uint32_t)SF_STAGES && !sf_wait(&b.empty[s], parity, b.abort)) return false;
+    tc::mbar_arrive_expect_tx(&b.full[s], SF_STAGE);
+    tc::tma_load_2d(stages + s * SF_STAGE, map, kb * 64, row, &b.full[s]);
+    ++*issued;
+    if (++s == SF_STAGES) s = 0, parity ^= 1;
+    return true;
+  };
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
-    for (int e = 0; e < 2 + 4 * SF_KB + nc * SF_KB; ++e) {
-      if (e == 2) {  // the input block, once the previous tile's output layer no longer reads A
-        if (local > 0 && !sf_wait(b.afree, (local - 1) & 1, b.abort)) return false;
-        tc::mbar_arrive_expect_tx(b.xfull, 128 * 128);
-        tc::tma_load_2d(abuf, tx, 0, tile * 128, b.xfull);
-        *xloads = local + 1;
-      }
-      const CUtensorMap* map;
-      int row, kb;
-      if (e < 2) {
-        map = tw1, row = 256 * e, kb = 0;
-      } else if (e < 2 + 4 * SF_KB) {
-        const int f = e - 2;  // layer (f / (2 KB)), then k-block, then half
-        map = f < 2 * SF_KB ? tw2 : tw3;
-        kb = (f % (2 * SF_KB)) / 2;
-        row = 256 * (f & 1);
-      } else {
-        const int f = e - 2 - 4 * SF_KB;  // chunk position, then k-block
-        map = tw4, row = 256 * ((f / SF_KB + blockIdx.x % nc) % nc), kb = f % SF_KB;
-      }
-      const uint32_t s = it % SF_STAGES;
-      if (it >= (uint32_t)SF_STAGES && !sf_wait(&b.empty[s], ((it / SF_STAGES) - 1) & 1, b.abort)) return false;
-      tc::mbar_arrive_expect_tx(&b.full[s], SF_STAGE);
-      tc::tma_load_2d(stages + s * SF_STAGE, map, kb * 64, row, &b.full[s]);
-      *issued = ++it;
+    if (!stage(tw1, 0, 0) || !stage(tw1, 0, 256)) return false;
+    // the input block, once the previous tile's output layer no longer reads A
+    if (local > 0 && !sf_wait(b.afree, (local - 1) & 1, b.abort)) return false;
+    tc::mbar_arrive_expect_tx(b.xfull, 128 * 128);
+    tc::tma_load_2d(abuf, tx, 0, tile * 128, b.xfull);
+    *xloads = local + 1;
+    for (int layer = 0; layer < 2; ++layer)
+      for (int kb = 0; kb < SF_KB; ++kb)
+        if (!stage(layer ? tw3 : tw2, kb, 0) || !stage(layer ? tw3 : tw2, kb, 256)) return false;
+    int c = blockIdx.x % nc;
+    for (int p = 0; p < nc; ++p) {
+      for (int kb = 0; kb < SF_KB; ++kb)
+        if (!stage(tw4, kb, 256 * c)) return false;
+      if (++c == nc) c = 0;
     }
   }
   return true;
 }
 
-// MMA issuer (one thread).
+// MMA issuer (one thread). What it does a stage stands between the stage's
+// MMAs and the next's, so descriptors and stage counters are kept, not formed.
 __device__ bool sf_mma(uint32_t tmem, uint32_t a0, uint8_t* stages, const SfBars& b, int tiles, int nc, int c0,
                        int c1) {
   const uint32_t idesc = tc::idesc_bf16(128, 256);
-  uint32_t it = 0, local = 0;
+  const uint64_t adesc = tc::sdesc_sw128(a0), bdesc = tc::sdesc_sw128(tc::smem_u32(stages));
+  uint32_t s = 0, parity = 0, local = 0;
+  auto stage = [&](uint32_t d, int kb) {  // the next weight stage against A's k-block kb
+    if (!sf_wait(&b.full[s], parity, b.abort)) return false;
+    tc::tc_fence_after();
+    const uint64_t ad = adesc + kb * (16384 >> 4), bd = bdesc + s * (SF_STAGE >> 4);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tc::mma_bf16(d, ad + 2 * k, bd + 2 * k, idesc, kb > 0 || k > 0 ? 1u : 0u);
+    tc::mma_commit(&b.empty[s]);
+    if (++s == SF_STAGES) s = 0, parity ^= 1;
+    return true;
+  };
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++local) {
     if (local > 0) {  // both slots drained by the previous tile's output epilogue
       if (c0 && !sf_wait(&b.accempty[0], (local * c0 - 1) & 1, b.abort)) return false;
@@ -174,48 +183,29 @@ __device__ bool sf_mma(uint32_t tmem, uint32_t a0, uint8_t* stages, const SfBars
     }
     if (!sf_wait(b.xfull, local & 1, b.abort)) return false;
     tc::tc_fence_after();
-    for (int e = 0; e < 2 + 4 * SF_KB + nc * SF_KB; ++e) {
-      uint32_t d, a;
-      bool first;
-      if (e < 2) {
-        d = tmem + 256 * e, a = a0, first = true;
-      } else if (e < 2 + 4 * SF_KB) {
-        const int f = e - 2;
-        if (f % (2 * SF_KB) == 0) {  // a new hidden layer: its A written and TMEM drained
-          if (!sf_wait(b.edone, (local * 3 + f / (2 * SF_KB)) & 1, b.abort)) return false;
-          tc::tc_fence_after();
-        }
-        const int kb = (f % (2 * SF_KB)) / 2;
-        d = tmem + 256 * (f & 1), a = a0 + kb * 16384, first = kb == 0;
-      } else {
-        const int f = e - 2 - 4 * SF_KB, c = f / SF_KB, kb = f % SF_KB, sl = c & 1;
-        if (f == 0) {  // the last hidden layer's activations are in A
-          if (!sf_wait(b.edone, (local * 3 + 2) & 1, b.abort)) return false;
-          tc::tc_fence_after();
-        }
-        if (kb == 0 && c >= 2) {  // chunk c - 2 of this slot drained
-          const uint32_t done = (sl ? local * c1 : local * c0) + (c - 2) / 2;
-          if (!sf_wait(&b.accempty[sl], done & 1, b.abort)) return false;
-          tc::tc_fence_after();
-        }
-        d = tmem + 256 * sl, a = a0 + kb * 16384, first = kb == 0;
+    for (int layer = 0; layer < 3; ++layer) {
+      if (layer > 0) {  // a new hidden layer: its A written and TMEM drained
+        if (!sf_wait(b.edone, (local * 3 + layer - 1) & 1, b.abort)) return false;
+        tc::tc_fence_after();
       }
-      const uint32_t s = it % SF_STAGES;
-      if (!sf_wait(&b.full[s], (it / SF_STAGES) & 1, b.abort)) return false;
-      tc::tc_fence_after();
-      const uint32_t bs = tc::smem_u32(stages + s * SF_STAGE);
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        tc::mma_bf16(d, tc::sdesc_sw128(a + 32 * k), tc::sdesc_sw128(bs + 32 * k), idesc, (!first || k > 0) ? 1u : 0u);
-      tc::mma_commit(&b.empty[s]);
-      ++it;
-      // accumulators complete: after layer 1, after each hidden layer, after each output chunk
-      if (e == 1 || (e >= 2 && e < 2 + 4 * SF_KB && (e - 2) % (2 * SF_KB) == 2 * SF_KB - 1)) {
-        tc::mma_commit(&b.accfull[0]);
-        tc::mma_commit(&b.accfull[1]);
-      } else if (e >= 2 + 4 * SF_KB && (e - 2 - 4 * SF_KB) % SF_KB == SF_KB - 1) {
-        tc::mma_commit(&b.accfull[((e - 2 - 4 * SF_KB) / SF_KB) & 1]);
+      const int blocks = layer == 0 ? 1 : SF_KB;
+      for (int kb = 0; kb < blocks; ++kb)
+        if (!stage(tmem, kb) || !stage(tmem + 256, kb)) return false;
+      tc::mma_commit(&b.accfull[0]);
+      tc::mma_commit(&b.accfull[1]);
+    }
+    if (!sf_wait(b.edone, (local * 3 + 2) & 1, b.abort)) return false;  // the last hidden activations are in A
+    tc::tc_fence_after();
+    for (int c = 0; c < nc; ++c) {
+      const int sl = c & 1;
+      if (c >= 2) {  // chunk c - 2 of this slot drained
+        const uint32_t done = (sl ? local * c1 : local * c0) + (c - 2) / 2;
+        if (!sf_wait(&b.accempty[sl], done & 1, b.abort)) return false;
+        tc::tc_fence_after();
       }
+      for (int kb = 0; kb < SF_KB; ++kb)
+        if (!stage(tmem + 256 * sl, kb)) return false;
+      tc::mma_commit(&b.accfull[sl]);
     }
     tc::mma_commit(b.afree);
   }
