@@ -29,10 +29,9 @@ void launch_lidar_segment(const Segments& g, int k, const LidarShape& shape, con
 void launch_lidar(const TrackDev& t, const float4* ray, float* obs, int n, int beams, const float2* beam_dir,
                   int* iters, cudaStream_t st);
 // Only the cars list[0 .. *list_count) (at most list_max; the count is read on the device): a
-// persistent grid pulling (car, beam group) units from `counter` (zeroed here). sms = SM count.
+// persistent grid striding over the (car, beam group) units. sms = SM count.
 void launch_lidar_list(const TrackDev& t, const float4* ray, float* obs, int n, int beams, const float2* beam_dir,
-                       const int* list, const int* list_count, int list_max, unsigned* counter, int sms,
-                       cudaStream_t st);
+                       const int* list, const int* list_count, int list_max, int sms, cudaStream_t st);
 bool lidar_shape_ok(const LidarShape& shape);
 // Spot check: beams (step % stride) + k stride of every car traced exactly and compared with the
 // predicted rows pred [beams, n]; cars off by more than tol (range / RANGE units) get minr = 0.

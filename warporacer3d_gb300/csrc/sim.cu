@@ -707,22 +707,13 @@ constexpr int lidar_min_blocks(int cars, bool wide) {
 // One track (cars [c0, c1) of the batch): its fields are kernel parameters,
 // read as constant operands. CARS warps per block (one car each): small
 // blocks release their slot as soon as their few cars finish.
-template <int LAYERS, int CARS, bool WIDE, bool LIST>
+template <int LAYERS, int CARS, bool WIDE>
 __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
     k_lidar_track(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0, int c1,
-                  int beams, const float2* __restrict__ beam_dir, int* iters, const int* __restrict__ list,
-                  const int* list_count) {
+                  int beams, const float2* __restrict__ beam_dir, int* iters) {
   early_start();
   const int beam = blockIdx.y * 32 + (threadIdx.x & 31);
   if (beam >= beams) return;
-  if (LIST) {  // only the listed cars (surrogate fallback), grid-stride over the list
-    const int count = *list_count;
-    for (int q = blockIdx.x * CARS + (threadIdx.x >> 5); q < count; q += gridDim.x * CARS) {
-      const int car = list[q];
-      if (car < n) trace<LAYERS>(t, ray, obs, n, beam_dir, max_iters, iters, car, beam);
-    }
-    return;
-  }
   const int car = c0 + (int)blockIdx.x * CARS + (int)(threadIdx.x >> 5);
   if (car < c1) trace<LAYERS>(t, ray, obs, n, beam_dir, max_iters, iters, car, beam);
 }
@@ -747,16 +738,12 @@ __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
 // (car, 32-beam group) units from `counter` (zero at launch) one at a time,
 // so no warp holds a block slot waiting for a sibling and the last wave has
 // no tail of idle slots.
-// With LIST, the cars are list[0 .. *list_count) (the surrogate's fallback
-// cars, counted on the device), whatever their number.
-template <int LAYERS, bool WIDE, bool LIST>
+template <int LAYERS, bool WIDE>
 __global__ void __launch_bounds__(128, lidar_min_blocks(4, WIDE))
     k_lidar_dynamic(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0, int c1,
-                    int beams, const float2* __restrict__ beam_dir, int* iters, unsigned* counter,
-                    const int* __restrict__ list, const int* list_count) {
+                    int beams, const float2* __restrict__ beam_dir, int* iters, unsigned* counter) {
   const int groups = (beams + 31) >> 5;
-  const unsigned cars = LIST ? (unsigned)min(max(*list_count, 0), n) : (unsigned)(c1 - c0);
-  const unsigned total = cars * (unsigned)groups;
+  const unsigned total = (unsigned)(c1 - c0) * (unsigned)groups;
   const int lane = threadIdx.x & 31;
   // the next unit is claimed before the current one is traced, so the atomic's
   // round trip overlaps the march
@@ -765,10 +752,28 @@ __global__ void __launch_bounds__(128, lidar_min_blocks(4, WIDE))
   unsigned unit = __shfl_sync(0xffffffffu, next, 0);
   while (unit < total) {
     if (lane == 0) next = atomicAdd(counter, 1u);
-    const int car = LIST ? list[unit / (unsigned)groups] : c0 + (int)(unit / (unsigned)groups);
+    const int car = c0 + (int)(unit / (unsigned)groups);
     const int beam = (int)(unit % (unsigned)groups) * 32 + lane;
     if (beam < beams && (unsigned)car < (unsigned)n) trace<LAYERS>(t, ray, obs, n, beam_dir, max_iters, iters, car, beam);
     unit = __shfl_sync(0xffffffffu, next, 0);
+  }
+}
+
+// The cars list[0 .. *list_count) alone (the surrogate's fallback cars, counted
+// on the device), whatever their number: a grid of all 64 warp slots an SM
+// whose warps stride over the (car, 32-beam group) units. About 3000 cars of
+// 1081 beams on the bridge take 95 us; 48 warps of 40 registers claiming their
+// units from a counter took 104, 64 that claim them 108.
+template <int LAYERS>
+__global__ void __launch_bounds__(128, lidar_min_blocks(4, false))
+    k_lidar_list(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int beams,
+                 const float2* __restrict__ beam_dir, const int* __restrict__ list, const int* list_count) {
+  const unsigned groups = (unsigned)(beams + 31) >> 5, total = (unsigned)min(max(*list_count, 0), n) * groups;
+  const unsigned warps = gridDim.x * (blockDim.x >> 5);
+  for (unsigned unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); unit < total; unit += warps) {
+    const int car = list[unit / groups], beam = (int)(unit % groups) * 32 + (int)(threadIdx.x & 31);
+    if (beam < beams && (unsigned)car < (unsigned)n)
+      trace<LAYERS>(t, ray, obs, n, beam_dir, max_iters, nullptr, car, beam);
   }
 }
 
@@ -1043,8 +1048,8 @@ static void lidar_track(const TrackDev& t, int max_iters, const float4* ray, flo
   }
   dim3 grid((c1 - c0 + CARS - 1) / CARS, (beams + 31) / 32);
   if (grid.x == 0) return;
-  lidar_launch(k_lidar_track<LAYERS, CARS, WIDE, false>, grid, CARS * 32, st, early, t, max_iters, ray, obs, n, c0, c1, beams,
-               beam_dir, iters, (const int*)nullptr, (const int*)nullptr);
+  lidar_launch(k_lidar_track<LAYERS, CARS, WIDE>, grid, CARS * 32, st, early, t, max_iters, ray, obs, n, c0, c1, beams,
+               beam_dir, iters);
 }
 
 template <int LAYERS, bool WIDE>
@@ -1055,8 +1060,8 @@ static void lidar_dynamic(const TrackDev& t, int max_iters, const float4* ray, f
   if (units <= 0) return;
   const long blocks = std::min<long>((long)sms * lidar_min_blocks(4, WIDE), (units + 3) / 4);
   cudaMemsetAsync(counter, 0, sizeof(unsigned), st);
-  k_lidar_dynamic<LAYERS, WIDE, false><<<(unsigned)blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, c0, c1, beams,
-                                                                          beam_dir, iters, counter, nullptr, nullptr);
+  k_lidar_dynamic<LAYERS, WIDE><<<(unsigned)blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, c0, c1, beams, beam_dir,
+                                                                  iters, counter);
 }
 
 template <int CARS, bool WIDE>
@@ -1171,23 +1176,17 @@ void launch_lidar(const TrackDev& t, const float4* ray, float* obs, int n, int b
 }
 
 void launch_lidar_list(const TrackDev& t, const float4* ray, float* obs, int n, int beams, const float2* beam_dir,
-                       const int* list, const int* list_count, int list_max, unsigned* counter, int sms,
-                       cudaStream_t st) {
+                       const int* list, const int* list_count, int list_max, int sms, cudaStream_t st) {
   const long units = (long)list_max * ((beams + 31) / 32);
   if (units <= 0) return;
-  // the 40-register variant: no spills with the list indirection
-  const long blocks = std::min<long>((long)sms * lidar_min_blocks(4, true), (units + 3) / 4);
+  const unsigned blocks = (unsigned)std::min<long>((long)sms * lidar_min_blocks(4, false), (units + 3) / 4);
   const int max_iters = lidar_max_iters(t);
-  cudaMemsetAsync(counter, 0, sizeof(unsigned), st);
   if (t.layers == 1)
-    k_lidar_dynamic<1, true, true><<<(unsigned)blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, 0, n, beams, beam_dir,
-                                                                     nullptr, counter, list, list_count);
+    k_lidar_list<1><<<blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, beams, beam_dir, list, list_count);
   else if (t.layers == 2)
-    k_lidar_dynamic<2, true, true><<<(unsigned)blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, 0, n, beams, beam_dir,
-                                                                     nullptr, counter, list, list_count);
+    k_lidar_list<2><<<blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, beams, beam_dir, list, list_count);
   else
-    k_lidar_dynamic<0, true, true><<<(unsigned)blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, 0, n, beams, beam_dir,
-                                                                     nullptr, counter, list, list_count);
+    k_lidar_list<0><<<blocks, 128, 0, st>>>(t, max_iters, ray, obs, n, beams, beam_dir, list, list_count);
 }
 
 // Spot check of a learned prediction: beams offset, offset + stride, ... of

@@ -811,7 +811,6 @@ struct racer_surrogate {
   unsigned* minr = nullptr;  // [n] smallest predicted range per car (uint bits)
   int* list = nullptr;       // [n] fallback cars
   int* list_count = nullptr;
-  unsigned* list_units = nullptr;  // unit counter of the fallback lidar
   float* exact = nullptr;    // [4 + beams, n] audit ranges
   double* rsums = nullptr;   // audit sum |e|, sum e^2 (metres)
   unsigned* rmax = nullptr;
@@ -1157,7 +1156,7 @@ int racer_surrogate_destroy(racer_surrogate* s) {
     cudaFree(p);
   free_acts(&s->train);
   free_acts(&s->infer);
-  for (void* p : {(void*)s->minr, (void*)s->list, (void*)s->list_count, (void*)s->list_units, (void*)s->exact,
+  for (void* p : {(void*)s->minr, (void*)s->list, (void*)s->list_count, (void*)s->exact,
                   (void*)s->rsums, (void*)s->rmax, (void*)s->rcount})
     cudaFree(p);
   delete s;
@@ -1289,10 +1288,10 @@ int racer_surrogate_bind(racer_surrogate* s, racer_sim* sim) {
   if (s->infer.M && s->infer.M != sim->n) {  // inference buffers are sized for the cars
     free_acts(&s->infer);
     s->infer = SurrogateActs();
-    for (void* p : {(void*)s->minr, (void*)s->list, (void*)s->list_count, (void*)s->list_units, (void*)s->exact,
+    for (void* p : {(void*)s->minr, (void*)s->list, (void*)s->list_count, (void*)s->exact,
                     (void*)s->wout})
       cudaFree(p);
-    s->minr = nullptr, s->list = nullptr, s->list_count = nullptr, s->list_units = nullptr, s->exact = nullptr;
+    s->minr = nullptr, s->list = nullptr, s->list_count = nullptr, s->exact = nullptr;
     s->wout = nullptr;
   }
   s->sim = sim;
@@ -1537,7 +1536,7 @@ int surrogate_prepare(racer_surrogate* s, racer_sim* sim) {
     if ((rc = salloc(&s->wout, (size_t)n * s->L.npad))) return rc;
   }
   if ((rc = make_acts(s, &s->infer, n, false)) || (rc = salloc(&s->minr, (size_t)n)) ||
-      (rc = salloc(&s->list, (size_t)n)) || (rc = salloc(&s->list_count, 1)) || (rc = salloc(&s->list_units, 1)) ||
+      (rc = salloc(&s->list, (size_t)n)) || (rc = salloc(&s->list_count, 1)) ||
       (rc = salloc(&s->exact, (size_t)(4 + sim->beams) * n)))
     return rc;
   if (!s->rsums && ((rc = salloc(&s->rsums, 2)) || (rc = salloc(&s->rmax, 1)) || (rc = salloc(&s->rcount, 2))))
@@ -1599,8 +1598,8 @@ int surrogate_lidar(racer_surrogate* s, racer_sim* sim, float* obs, bool audit, 
     SURR_CHECK(cudaMemsetAsync(s->list_count, 0, sizeof(int), st));
     // the threshold stays above 0 so that marked cars are always selected
     launch_select_cars(s->minr, n, fallback > 0.0f ? fallback : 1e-30f, s->list, s->list_count, st);
-    launch_lidar_list(sim->t, sim->ray, obs, n, beams, sim->beam_dir, s->list, s->list_count, n, s->list_units,
-                      sim->sms, st);
+    launch_lidar_list(sim->t, sim->ray, obs, n, beams, sim->beam_dir, s->list, s->list_count, n, sim->sms,
+                      st);
     k_count_fallback<<<1, 32, 0, st>>>(s->list_count, s->rcount + 1);
   }
   if (audit) k_compare<<<1216, 256, 0, st>>>(pred, obs + 4L * n, (long)beams * n, s->rsums, s->rmax, s->rcount);
