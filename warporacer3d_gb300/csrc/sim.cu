@@ -1219,9 +1219,16 @@ __global__ void k_lidar_spot(TrackDev t, int max_iters, const float4* __restrict
 // physics of each car (one thread each), the lidar (a warp marches 32 beams of
 // one car at a time). Cars never interact, so no grid-wide synchronisation is
 // needed, and every result is the chained graph's: the same device functions
-// (advance_car, trace) and the same forward (k-blocks, MMAs, epilogue) as
+// (advance_car, beam_range) and the same forward (k-blocks, MMAs, epilogue) as
 // mlp_tc.cu's register-staged kernel. Two CTAs share an SM, so one's forward or
 // physics, latency-bound, runs beside the other's lidar.
+// A CTA has few cars (4 of 1024 on 152 SMs), so a step is a chain of
+// latencies. RESIDENT (inputs of at most GROUPS k-blocks, 128): the weights
+// stay in shared memory, and each beam's range goes from the march straight to
+// its place in the next step's A operand, so that the forward loads nothing.
+// Wider inputs take their k-blocks through the stages, a row in parts by
+// several threads. 100 steps of 1024 cars x 108 beams: 2033 us against 2322 with
+// a thread a row and four round trips to L2 for each k-block.
 // Data the kernel rewrites every step (obs, the ray frames, actions) is read
 // with coherent loads (never the read-only path); the block's barrier orders
 // its writes before the next phase's reads.
@@ -1240,7 +1247,13 @@ struct FusedRolloutCfg {
 };
 static_assert(2 * FusedRolloutCfg::SMEM_BYTES <= 227 * 1024, "two CTAs per SM");
 
-template <int LAYERS>
+// Input f of a tile's row in the A stages, as the MMAs read it.
+__device__ __forceinline__ __nv_bfloat16* fused_input(uint8_t* A, int row, int f) {
+  return reinterpret_cast<__nv_bfloat16*>(A + (f >> 6) * A_BYTES + row * 128 +
+                                          ((((f & 63) >> 3) ^ (row & 7)) << 4)) + (f & 7);
+}
+
+template <int LAYERS, bool RESIDENT>
 __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
     k_rollout_fused(const __grid_constant__ Segments g, float* s, float* act, float* reward, float* done_rows,
                     float* obs, int n, int beams, float4* ray, const float2* __restrict__ beam_dir, int cars_per_cta,
@@ -1286,6 +1299,16 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
     for (int e = tid; e < 2 * B_BYTES / 16; e += C::THREADS) w1[e] = __ldg(w1s + e);
     for (int e = tid; e < 2 * 16 * 128 / 16; e += C::THREADS) w2[e] = __ldg(w2s + e);
   }
+  if (RESIDENT) {  // W0, and the first step's inputs; rows past the CTA's cars meet nothing that is used
+    uint4* w0 = reinterpret_cast<uint4*>(smem + C::OFF_B);
+    for (int e = tid; e < kblocks * (B_BYTES / 16); e += C::THREADS) w0[e] = __ldg(w0s + e);
+    const int cars = c1 - c0;
+    for (int e = tid; e < cars * kblocks * 64; e += C::THREADS) {
+      const int row = e % cars, f = e / cars;
+      *fused_input(smem + C::OFF_A, row, f) =
+          __float2bfloat16_rn(f < in ? __ldcg(obs + (long)f * n + c0 + row) : 0.0f);
+    }
+  }
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
   __syncthreads();
@@ -1300,7 +1323,20 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
     // ---- policy forward on the cars' observations, with the sampling in the epilogue ----
     const int c = c0 + r;
     const bool live = c < c1;
-    if (warp < MMA_WARP) {
+    if (RESIDENT) {
+      if (warp == MMA_WARP && lane == 0 && !*abort) {
+        issued = true;
+        tc::tc_fence_after();
+        for (int kb = 0; kb < kblocks; ++kb) {
+          const uint32_t a = tc::smem_u32(smem + C::OFF_A + kb * A_BYTES);
+          const uint32_t b = tc::smem_u32(smem + C::OFF_B + kb * B_BYTES);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            tc::mma_bf16(tmem, tc::sdesc_sw128(a + 32 * k), tc::sdesc_sw128(b + 32 * k), id64, (kb | k) ? 1u : 0u);
+        }
+        tc::mma_commit(done);
+      }
+    } else if (warp < MMA_WARP) {
       const int q = warp >> 2;                               // producer group: k-blocks q, q + GROUPS, ...
       const uint32_t uses = (kblocks - q + GROUPS - 1) / GROUPS;  // uses of its stage in a step
       uint8_t* A = smem + C::OFF_A + q * A_BYTES;
@@ -1314,23 +1350,24 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
 #pragma unroll
         for (int e = 0; e < 4; ++e) wb[e] = __ldg(src + r + e * TILE);
         if (use >= 1 && !tc::mbar_wait_abort(&empty[q], (use - 1) & 1, abort, limit)) ok = false;
-        // the k-block's 64 inputs of this row in four chunks of 16 (the same BF16 operand as mlp_tc.cu's
-        // producers write; fewer live registers)
+        // 8 inputs of 32 rows at a time, two rows a thread (the same BF16 operand as mlp_tc.cu's producers write);
+        // rows past the CTA's cars meet nothing that is used
+        const int chunk = r >> 4;
 #pragma unroll 1
-        for (int h = 0; h < 4; ++h) {
-          float v[16];
+        for (int row = r & 15; row < c1 - c0; row += 32) {
+          float v[2][8];
 #pragma unroll
-          for (int f = 0; f < 16; ++f) {
-            const int row = kb * 64 + 16 * h + f;
-            v[f] = (live && row < in) ? __ldcg(obs + (long)row * n + c) : 0.0f;
-          }
+          for (int y = 0; y < 2; ++y)
 #pragma unroll
-          for (int f = 0; f < 2; ++f) {
-            const int chunk = 2 * h + f;
-            const uint4 pk = make_uint4(tc::pack_bf16(v[8 * f], v[8 * f + 1]), tc::pack_bf16(v[8 * f + 2], v[8 * f + 3]),
-                                        tc::pack_bf16(v[8 * f + 4], v[8 * f + 5]),
-                                        tc::pack_bf16(v[8 * f + 6], v[8 * f + 7]));
-            *reinterpret_cast<uint4*>(A + r * 128 + ((chunk ^ (r & 7)) << 4)) = pk;
+            for (int f = 0; f < 8; ++f) {
+              const int i = kb * 64 + 8 * chunk + f;
+              v[y][f] = c0 + row + 16 * y < c1 && i < in ? __ldcg(obs + (long)i * n + c0 + row + 16 * y) : 0.0f;
+            }
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {  // row + 16 has row's swizzle
+            const uint4 pk = make_uint4(tc::pack_bf16(v[y][0], v[y][1]), tc::pack_bf16(v[y][2], v[y][3]),
+                                        tc::pack_bf16(v[y][4], v[y][5]), tc::pack_bf16(v[y][6], v[y][7]));
+            *reinterpret_cast<uint4*>(A + (row + 16 * y) * 128 + ((chunk ^ (row & 7)) << 4)) = pk;
           }
         }
 #pragma unroll
@@ -1372,7 +1409,24 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
     const int units = (c1 - c0) * beam_groups;
     for (int u = warp; u < units; u += C::THREADS / 32) {
       const int car = c0 + u / beam_groups, beam = (u % beam_groups) * 32 + lane;
-      if (beam < beams) trace<LAYERS, false>(t, ray, obs, n, beam_dir, g.max_iters[0], nullptr, car, beam);
+      if (beam >= beams) continue;
+      if (RESIDENT) {
+        int count;
+        const float v = range_obs(beam_range<LAYERS, false>(t, ray, n, beam_dir, g.max_iters[0], false, car, beam, &count));
+        obs[(long)(4 + beam) * n + car] = v;
+        *fused_input(smem + C::OFF_A, car - c0, 4 + beam) = __float2bfloat16_rn(v);
+      } else {
+        trace<LAYERS, false>(t, ray, obs, n, beam_dir, g.max_iters[0], nullptr, car, beam);
+      }
+    }
+    if (RESIDENT) {  // the other inputs, and zeros to the k-block's end, where the forward left its activations
+      const int cars = c1 - c0, others = kblocks * 64 - beams;
+      for (int e = tid; e < cars * others; e += C::THREADS) {
+        const int row = e % cars, j = e / cars, f = j < 4 ? j : beams + j;
+        *fused_input(smem + C::OFF_A, row, f) =
+            __float2bfloat16_rn(f < in ? __ldcg(obs + (long)f * n + c0 + row) : 0.0f);
+      }
+      tc::fence_proxy_async_smem();
     }
     tc::tc_fence_before();
     __syncthreads();  // obs complete before the next step's forward reads it
@@ -1430,7 +1484,8 @@ cudaError_t launch_rollout_fused(const Segments& g, float* state, float* actions
                                  cudaStream_t st) {
   static unsigned long long configured = 0;  // per device
   cudaError_t e = once_per_device(&configured, [] {
-    for (auto* k : {k_rollout_fused<0>, k_rollout_fused<1>, k_rollout_fused<2>}) {
+    for (auto* k : {k_rollout_fused<0, false>, k_rollout_fused<1, false>, k_rollout_fused<2, false>,
+                    k_rollout_fused<0, true>, k_rollout_fused<1, true>, k_rollout_fused<2, true>}) {
       cudaError_t a = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedRolloutCfg::SMEM_BYTES);
       if (a != cudaSuccess) return a;
     }
@@ -1446,7 +1501,8 @@ cudaError_t launch_rollout_fused(const Segments& g, float* state, float* actions
   const unsigned blocks = (unsigned)((n + per - 1) / per);
   const int layers = g.t[0].layers;
 #define RACER_FUSED(L)                                                                                              \
-  k_rollout_fused<L><<<blocks, FusedRolloutCfg::THREADS, FusedRolloutCfg::SMEM_BYTES, st>>>(                        \
+  (kb <= FusedRolloutCfg::GROUPS ? k_rollout_fused<L, true> : k_rollout_fused<L, false>)                              \
+      <<<blocks, FusedRolloutCfg::THREADS, FusedRolloutCfg::SMEM_BYTES, st>>>(                                      \
       g, state, actions, reward, done, obs, n, beams, ray, beam_dir, per, steps, w0, kb, w1, w2, og, sa, err)
   if (layers == 1)
     RACER_FUSED(1);
