@@ -162,19 +162,25 @@ __global__ void __launch_bounds__(128, 4)
 // m is the weight's input index, column n its output row). One warp per
 // element: lane l sums the partials z = l, l + 32, ... in order, then a fixed
 // shuffle tree adds the lanes (deterministic).
-__global__ void k_wgrad_reduce(const float* __restrict__ P, int splits, int mrows, int nreal, int mreal,
-                               float* grad, int ldg) {
-  const long total = (long)mreal * nreal;
-  const int lane = threadIdx.x & 31;
-  const long warps = ((long)gridDim.x * blockDim.x) >> 5;
-  for (long e = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; e < total; e += warps) {
-    const int m = (int)(e / nreal), n = (int)(e % nreal);
-    float acc = 0.0f;
-    for (int z = lane; z < splits; z += 32) acc += P[((long)z * mrows + m) * nreal + n];
-#pragma unroll
-    for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if (lane == 0) grad[(long)n * ldg + m] = acc;
+constexpr int RED_ELEMENTS = 32;
+__global__ void __launch_bounds__(RED_ELEMENTS * 32) k_wgrad_reduce(const float* __restrict__ P, int splits, int mrows,
+                                                                    int nreal, int mreal, float* grad, int ldg) {
+  __shared__ float sums[32][RED_ELEMENTS + 1];
+  const int total = mreal * nreal, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int e = (int)blockIdx.x * RED_ELEMENTS + lane;
+  float acc = 0.0f;
+  if (e < total) {
+    const float* p = P + e;  // element (m, n) of a partial is at m nreal + n = e
+#pragma unroll 4
+    for (int z = warp; z < splits; z += 32) acc += __ldcs(p + (long)z * mrows * nreal);
   }
+  sums[warp][lane] = acc;
+  __syncthreads();
+  acc = sums[lane][warp];
+#pragma unroll
+  for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+  const int o = (int)blockIdx.x * RED_ELEMENTS + warp, m = o / nreal, n = o % nreal;
+  if (lane == 0 && o < total) grad[(long)n * ldg + m] = acc;
 }
 
 template <typename T>
@@ -249,9 +255,8 @@ int wgrad(BackwardWork* w, const CUtensorMap& ta, const CUtensorMap& tb, int mro
   splits = (kblocks + per - 1) / per;
   EpiSplitF32 epi{w->scratch, (long)mrows * nreal, mrows, nreal};
   BW_CHECK(gemm_launch<BN>(ta, tb, mrows, nreal, kblocks, splits, epi, err, st));
-  const long total = (long)mreal * nreal;
-  k_wgrad_reduce<<<(unsigned)std::min<long>((total + 7) / 8, 4096), 256, 0, st>>>(w->scratch, splits, mrows, nreal,
-                                                                                     mreal, grad, ldg);
+  k_wgrad_reduce<<<(mreal * nreal + RED_ELEMENTS - 1) / RED_ELEMENTS, RED_ELEMENTS * 32, 0, st>>>(
+      w->scratch, splits, mrows, nreal, mreal, grad, ldg);
   BW_CHECK(cudaGetLastError());
   return 0;
 }
