@@ -89,6 +89,8 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
+  early_next();  // not before the TMEM is allocated: a CTA that waits for this kernel must not hold what this one needs
+  early_wait();
 
   if (warp == 0 && lane == 0) {
     uint32_t it = 0;
@@ -199,7 +201,7 @@ cudaError_t gemm_configure() {
 // boxes: K-contiguous operands 64 x 128 (A) and 64 x BN (B); MN ones 64 x 64.
 template <int BN, typename Epi, bool MN = false>
 cudaError_t gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int N, int kblocks, int splits,
-                        const Epi& epi, int* err, cudaStream_t st) {
+                        const Epi& epi, int* err, cudaStream_t st, bool early = false) {
   using C = GemmCfg<BN>;
   cudaError_t ce = gemm_configure<BN, Epi, MN>();
   if (ce != cudaSuccess) return ce;
@@ -209,9 +211,8 @@ cudaError_t gemm_launch(const CUtensorMap& ta, const CUtensorMap& tb, int M, int
   splits = (kblocks + per - 1) / per;
   const int mtiles = (M + C::BM - 1) / C::BM, ntiles = (N + BN - 1) / BN;
   const int tiles = mtiles * ntiles * splits;
-  k_gemm<BN, Epi, MN><<<tiles < sms ? tiles : sms, C::THREADS, C::SMEM, st>>>(ta, tb, mtiles, ntiles, splits, kblocks,
-                                                                              per, epi, err);
-  return cudaGetLastError();
+  return launch_early_if(early, k_gemm<BN, Epi, MN>, dim3(tiles < sms ? tiles : sms), C::THREADS, C::SMEM, st, ta, tb,
+                         mtiles, ntiles, splits, kblocks, per, epi, err);
 }
 
 }  // namespace

@@ -648,6 +648,7 @@ __global__ void k_rk4_f64(const __grid_constant__ Segments g, const float* prev,
 // the slopes along and across the heading, and the same frame k_advance
 // writes. Used to label surrogate training poses with the exact tracer.
 __global__ void k_pose_frames(TrackDev t, const float4* __restrict__ poses, int count, float4* ray) {
+  early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 p = poses[i];
@@ -1526,7 +1527,7 @@ void launch_rk4_audit(const Segments& g, const float* prev, const float* actions
 }
 
 void launch_pose_frames(const TrackDev& t, const float4* poses, int count, float4* ray, cudaStream_t st) {
-  k_pose_frames<<<(count + 127) / 128, 128, 0, st>>>(t, poses, count, ray);
+  launch_early(k_pose_frames, dim3((count + 127) / 128), 128, 0, st, t, poses, count, ray);
 }
 
 void launch_sample(int n, uint64_t seed, const float* output, const float* log_std, float* actions, float* logp,

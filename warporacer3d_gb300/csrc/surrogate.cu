@@ -368,6 +368,7 @@ __device__ __forceinline__ void store_inputs(const float* f, int i, bf16* x) {
 }
 
 __global__ void k_features(const float4* __restrict__ ray, int count, Norm nm, bf16* x) {
+  early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 r0 = ray[i], r1 = ray[count + i];
@@ -407,6 +408,7 @@ __device__ __forceinline__ void grid_features(const GridGeom& gg, const float* _
 //   56..63  sin/cos(2^k pi x'), sin/cos(2^k pi y') for k = 0, 1
 __global__ void k_features_cargrid(const float4* __restrict__ ray, int count, Norm nm, GridGeom gg,
                                    const float* __restrict__ grid, bf16* x) {
+  early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 r0 = ray[i], r1 = ray[count + i];
@@ -439,6 +441,7 @@ __global__ void k_features_cargrid(const float4* __restrict__ ray, int count, No
 //   62, 63  sin/cos(2 pi phase)
 __global__ void k_features_world(const float4* __restrict__ ray, int count, Norm nm, GridGeom gg,
                                  const float* __restrict__ grid, int K, bf16* x) {
+  early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   const float4 r0 = ray[i], r1 = ray[count + i];
@@ -470,6 +473,7 @@ __global__ void k_features_world(const float4* __restrict__ ray, int count, Norm
 // world samples out (the loss epilogue reads whole rows; reading the labels from there took a 32-byte sector a value).
 __global__ void __launch_bounds__(256) k_world_targets(const float* __restrict__ target, const float4* __restrict__ ray,
                                                        int B, int beams, int K, int ld, float* rows, int* k0) {
+  early_start();
   __shared__ float tile[32][33];
   __shared__ int first[32];
   const int lane = threadIdx.x & 31, row = threadIdx.x >> 5, m0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
@@ -498,6 +502,7 @@ __global__ void __launch_bounds__(256) k_world_targets(const float* __restrict__
 // four corners of its cell at every level (16-byte atomic adds).
 __global__ void k_grid_grad(const float4* __restrict__ ray, int B, GridGeom gg, const float* __restrict__ dx,
                             float* ggrad) {
+  early_start();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= B) return;
   const float4 r0 = ray[m], r1 = ray[B + m];
@@ -608,6 +613,7 @@ __global__ void k_sample_poses(const int2* cells, int ncells, int count, uint64_
 
 // Sum of split-K partials into a row-major gradient block of `count` floats (a multiple of 4), four per thread.
 __global__ void k_reduce_splits(const float* __restrict__ P, int splits, long mn, long count, float* out) {
+  early_start();
   const long e = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
   if (e >= count) return;
   float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -666,6 +672,7 @@ __global__ void k_refresh(const float* __restrict__ th, Layout L, bf16* w1b, bf1
 // What a gradient adds up in place, at zero: the biases' gradients (b4 and the feature grids lie at the end) and the
 // loss sums.
 __global__ void k_zero_sums(float* grad, Layout L, double* sums) {
+  early_start();
   const long i0 = (long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long)gridDim.x * blockDim.x;
   for (long i = i0; i < L.H; i += stride) grad[L.b2 + i] = grad[L.b3 + i] = 0.0f;
   const long quads = (L.total - L.b4) / 4;  // b4 is a multiple of 4
@@ -873,16 +880,19 @@ void free_acts(SurrogateActs* a) {
     }                                                                                     \
   } while (0)
 
-// Forward of M rows already featurised in a->x; the last layer uses `out` (inference).
+// Forward of M rows already featurised in a->x; the last layer uses `out` (inference). The kernels of a training batch
+// start early, each behind the one before it (8192 poses: 326 us a gradient without, 275 with); a rollout's do not, whose
+// waiting blocks would hold other streams' places (7.70 ms against 7.61 with the features' kernel alone early).
 int forward(racer_surrogate* s, SurrogateActs* a, const EpiInfer* out) {
   const int H = s->L.H, M = a->M;
   const float* th = s->theta;
   cudaStream_t st = s->st;
-  SURR_CHECK(gemm_launch<256>(a->tx, s->tw1, M, H, 1, 1, EpiTanhOut{a->h1s, H, nullptr, M, H}, s->err, st));
+  const bool early = a->g4s != nullptr;  // a training batch's
+  SURR_CHECK(gemm_launch<256>(a->tx, s->tw1, M, H, 1, 1, EpiTanhOut{a->h1s, H, nullptr, M, H}, s->err, st, early));
   SURR_CHECK(gemm_launch<256>(a->th1, s->tw2, M, H, H / 64, 1,
-                              EpiTanhOut{a->h2s, H, th + s->L.b2, M, H}, s->err, st));
+                              EpiTanhOut{a->h2s, H, th + s->L.b2, M, H}, s->err, st, early));
   SURR_CHECK(gemm_launch<256>(a->th2, s->tw3, M, H, H / 64, 1,
-                              EpiTanhOut{a->h3s, H, th + s->L.b3, M, H}, s->err, st));
+                              EpiTanhOut{a->h3s, H, th + s->L.b3, M, H}, s->err, st, early));
   if (out) SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, M, s->L.beams, H / 64, 1, *out, s->err, st));
   return 0;
 }
@@ -927,22 +937,24 @@ int wgrad(racer_surrogate* s, const CUtensorMap& ta, const CUtensorMap& tb, int 
     return 1;
   }
   EpiSplitF32 epi{s->scratch, (long)Mpad * N, Mpad, N};
-  SURR_CHECK((gemm_launch<BN, EpiSplitF32, true>(ta, tb, Mpad, N, kblocks, splits, epi, s->err, s->st)));
+  SURR_CHECK((gemm_launch<BN, EpiSplitF32, true>(ta, tb, Mpad, N, kblocks, splits, epi, s->err, s->st, true)));
   long count = (long)Mreal * N;
-  k_reduce_splits<<<(unsigned)((count / 4 + 127) / 128), 128, 0, s->st>>>(s->scratch, splits, (long)Mpad * N, count,
-                                                                          s->grad + off);
+  launch_early(k_reduce_splits, dim3((unsigned)((count / 4 + 127) / 128)), 128, 0, s->st, s->scratch, splits,
+               (long)Mpad * N, count, s->grad + off);
   SURR_CHECK(cudaGetLastError());
   return 0;
 }
 
 // Encoded inputs x [count, 64] of `count` ray frames.
-int featurise(racer_surrogate* s, const float4* ray, int count, bf16* x, cudaStream_t st) {
+int featurise(racer_surrogate* s, const float4* ray, int count, bf16* x, cudaStream_t st, bool early) {
   if (s->L.world)
-    k_features_world<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, s->gg, s->theta + s->L.g, s->L.nout, x);
+    launch_early_if(early, k_features_world, dim3((count + 127) / 128), 128, 0, st, ray, count, s->nm, s->gg,
+                    s->theta + s->L.g, s->L.nout, x);
   else if (s->L.grid)
-    k_features_cargrid<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, s->gg, s->theta + s->L.g, x);
+    launch_early_if(early, k_features_cargrid, dim3((count + 127) / 128), 128, 0, st, ray, count, s->nm, s->gg,
+                    s->theta + s->L.g, x);
   else
-    k_features<<<(count + 127) / 128, 128, 0, st>>>(ray, count, s->nm, x);
+    launch_early_if(early, k_features, dim3((count + 127) / 128), 128, 0, st, ray, count, s->nm, x);
   SURR_CHECK(cudaGetLastError());
   return 0;
 }
@@ -965,7 +977,7 @@ int prepare(racer_surrogate* s, SurrogateActs* a, long first, const float** labe
     if (keep) s->lcached[b] = 1;
   }
   *labels = slot;
-  return featurise(s, s->ray, B, a->x, s->st);
+  return featurise(s, s->ray, B, a->x, s->st, true);
 }
 
 // Gradient of the mean squared error over the batch into s->grad; loss sums into s->sums.
@@ -975,37 +987,38 @@ int gradient(racer_surrogate* s, long first, const float** labels) {
   int rc = prepare(s, a, first, labels, true);
   if (rc) return rc;
   const int nout = s->L.nout;
-  k_zero_sums<<<device_sms(), 256, 0, s->st>>>(s->grad, s->L, s->sums);
+  launch_early(k_zero_sums, dim3(device_sms()), 256, 0, s->st, s->grad, s->L, s->sums);
   SURR_CHECK(cudaGetLastError());
   if ((rc = forward(s, a, nullptr))) return rc;
   const float scale = 2.0f / ((float)B * (float)beams);
   LossSums losses;
   losses.sums = s->sums;
   if (s->L.world) {
-    k_world_targets<<<dim3((B + 31) / 32, (beams + 31) / 32), 256, 0, s->st>>>(*labels, s->ray, B, beams, nout,
-                                                                               NP, s->wtarget, s->wk0);
+    launch_early(k_world_targets, dim3((B + 31) / 32, (beams + 31) / 32), 256, 0, s->st, *labels, s->ray, B, beams,
+                 nout, NP, s->wtarget, s->wk0);
     SURR_CHECK(cudaGetLastError());
     EpiLoss<true> loss{s->wtarget, 0, s->wk0, beams, s->theta + s->L.b4, B, nout, scale, a->g4s, NP,
                        s->grad + s->L.b4, s->huber, losses};
-    SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, loss, s->err, s->st));
+    SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, loss, s->err, s->st, true));
   } else {
     EpiLoss<false> loss{*labels, B, nullptr, beams, s->theta + s->L.b4, B, beams, scale, a->g4s, NP,
                         s->grad + s->L.b4, s->huber, losses};
-    SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, loss, s->err, s->st));
+    SURR_CHECK(gemm_launch<256>(a->th3, s->tw4, B, NP, H / 64, 1, loss, s->err, s->st, true));
   }
   SURR_CHECK(gemm_launch<256>(a->tg4s, s->tw4t, B, H, NP / 64, 1,
-                              EpiDTanh{a->h3s, H, a->g3s, H, s->grad + s->L.b3, B, H}, s->err, s->st));
+                              EpiDTanh{a->h3s, H, a->g3s, H, s->grad + s->L.b3, B, H}, s->err, s->st, true));
   SURR_CHECK(gemm_launch<256>(a->tg3s, s->tw3t, B, H, H / 64, 1,
-                              EpiDTanh{a->h2s, H, a->g2s, H, s->grad + s->L.b2, B, H}, s->err, s->st));
+                              EpiDTanh{a->h2s, H, a->g2s, H, s->grad + s->L.b2, B, H}, s->err, s->st, true));
   SURR_CHECK(gemm_launch<256>(a->tg2s, s->tw2t, B, H, H / 64, 1, EpiDTanh{a->h1s, H, a->g1s, H, nullptr, B, H}, s->err,
-                              s->st));
+                              s->st, true));
   if ((rc = wgrad<256>(s, a->wg4, a->wh3, NP, nout, H, s->L.w4))) return rc;
   if ((rc = wgrad<256>(s, a->wg3, a->wh2, H, H, H, s->L.w3))) return rc;
   if ((rc = wgrad<256>(s, a->wg2, a->wh1, H, H, H, s->L.w2))) return rc;
   if ((rc = wgrad<64>(s, a->wg1, a->wx, H, H, NIN, s->L.w1))) return rc;
   if (s->L.grid) {  // dL/df = g1 W1, then onto the grids
-    SURR_CHECK(gemm_launch<64>(a->tg1s, s->tw1t, B, NIN, H / 64, 1, EpiRowF32{s->dx, NIN, B, NIN}, s->err, s->st));
-    k_grid_grad<<<B / 128, 128, 0, s->st>>>(s->ray, B, s->gg, s->dx, s->grad + s->L.g);
+    SURR_CHECK(gemm_launch<64>(a->tg1s, s->tw1t, B, NIN, H / 64, 1, EpiRowF32{s->dx, NIN, B, NIN}, s->err, s->st,
+                               true));
+    launch_early(k_grid_grad, dim3(B / 128), 128, 0, s->st, s->ray, B, s->gg, s->dx, s->grad + s->L.g);
     SURR_CHECK(cudaGetLastError());
   }
   return 0;
@@ -1560,7 +1573,7 @@ int surrogate_lidar(racer_surrogate* s, racer_sim* sim, float* obs, bool audit, 
                     const int64_t* step_base, int64_t step_add) {
   const int n = sim->n, beams = sim->beams;
   SurrogateActs* a = &s->infer;
-  if (int rc = featurise(s, sim->ray, n, a->x, st)) return rc;
+  if (int rc = featurise(s, sim->ray, n, a->x, st, false)) return rc;
   SURR_CHECK(cudaMemsetAsync(s->minr, 0x7f, (size_t)n * sizeof(unsigned), st));
   // on an audit step the prediction goes to the scratch rows and the exact tracer writes obs
   float* pred = audit ? s->exact + 4L * n : obs + 4L * n;
