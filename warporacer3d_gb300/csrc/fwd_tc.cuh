@@ -62,8 +62,10 @@ __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, u
                               tc::pack_bf16(acc[8 * q + 4], acc[8 * q + 5]),
                               tc::pack_bf16(acc[8 * q + 6], acc[8 * q + 7]));
         *reinterpret_cast<uint4*>(Hs + r * 128 + ((q ^ (r & 7)) << 4)) = pk;
-        uint4 hi = q == 0 ? make_uint4(tc::pack_bf16(1.0f, 0.0f), 0u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(Hs + A_BYTES + r * 128 + ((q ^ (r & 7)) << 4)) = hi;
+        if (q < 2) {  // the bias's one and 15 zeros: the only step of 16 k's past h
+          const uint4 hi = make_uint4(q == 0 ? tc::pack_bf16(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
+          *reinterpret_cast<uint4*>(Hs + A_BYTES + r * 128 + ((q ^ (r & 7)) << 4)) = hi;
+        }
       }
       if (write_hidden && live) {
         float* hg = layer == 0 ? h1g : h2g;
@@ -77,15 +79,13 @@ __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, u
       if (tid == 0 && !*abort) {
         *issued = true;
         tc::tc_fence_after();
-        const uint32_t h = tc::smem_u32(Hs);
-        const uint32_t w = tc::smem_u32(smem + (layer == 0 ? OFF_W1 : OFF_W2));
+        const uint64_t h = tc::sdesc_sw128(tc::smem_u32(Hs));
+        const uint64_t w = tc::sdesc_sw128(tc::smem_u32(smem + (layer == 0 ? OFF_W1 : OFF_W2)));
         const uint32_t wstride = layer == 0 ? B_BYTES : 16 * 128;
+        const uint32_t id = layer == 0 ? id64 : id16;
 #pragma unroll
-        for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            tc::mma_bf16(tmem, tc::sdesc_sw128(h + kb * A_BYTES + 32 * k),
-                         tc::sdesc_sw128(w + kb * wstride + 32 * k), layer == 0 ? id64 : id16, (kb | k) ? 1u : 0u);
+        for (int k = 0; k < 4; ++k) tc::mma_bf16(tmem, h + 2 * k, w + 2 * k, id, k ? 1u : 0u);
+        tc::mma_bf16(tmem, h + (A_BYTES >> 4), w + (wstride >> 4), id, 1u);
         tc::mma_commit(done);
       }
       if (!tc::mbar_wait_abort(done, (p0 + 1 + layer) & 1, abort, limit)) ok = false;

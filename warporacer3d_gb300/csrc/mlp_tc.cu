@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
       if (*abort) continue;  // issue nothing after a timeout
       issued = true;
       tc::tc_fence_after();
-      const uint32_t a = tc::smem_u32(smem + OFF_A + g * A_BYTES), b = tc::smem_u32(smem + OFF_B + g * B_BYTES);
+      const uint64_t ad = tc::sdesc_sw128(tc::smem_u32(smem + OFF_A + g * A_BYTES));
+      const uint64_t bd = tc::sdesc_sw128(tc::smem_u32(smem + OFF_B + g * B_BYTES));
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        tc::mma_bf16(tmem, tc::sdesc_sw128(a + 32 * k), tc::sdesc_sw128(b + 32 * k), id64, (kb | k) ? 1u : 0u);
+      for (int k = 0; k < 4; ++k) tc::mma_bf16(tmem, ad + 2 * k, bd + 2 * k, id64, (kb | k) ? 1u : 0u);
       tc::mma_commit(&empty[g]);
     }
     if (!*abort) tc::mma_commit(done);
@@ -305,11 +305,11 @@ __global__ void __launch_bounds__(TmaCfg::THREADS, 1)
           if (*abort) continue;  // issue nothing after a timeout
           issued = true;
           tc::tc_fence_after();
-          const uint32_t sa_ = tc::smem_u32(smem + C::OFF_A + a * A_BYTES);
-          const uint32_t sb = tc::smem_u32(smem + C::OFF_B + a * B_BYTES);
+          const uint64_t ad = tc::sdesc_sw128(tc::smem_u32(smem + C::OFF_A + a * A_BYTES));
+          const uint64_t bd = tc::sdesc_sw128(tc::smem_u32(smem + C::OFF_B + a * B_BYTES));
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            tc::mma_bf16(tmem, tc::sdesc_sw128(sa_ + 32 * k), tc::sdesc_sw128(sb + 32 * k), id64, (kb | k) ? 1u : 0u);
+            tc::mma_bf16(tmem, ad + 2 * k, bd + 2 * k, id64, (kb | k) ? 1u : 0u);
           tc::mma_commit(&aempty[a]);
         }
         if (!*abort) tc::mma_commit(done);

@@ -1329,11 +1329,10 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
         issued = true;
         tc::tc_fence_after();
         for (int kb = 0; kb < kblocks; ++kb) {
-          const uint32_t a = tc::smem_u32(smem + C::OFF_A + kb * A_BYTES);
-          const uint32_t b = tc::smem_u32(smem + C::OFF_B + kb * B_BYTES);
+          const uint64_t a = tc::sdesc_sw128(tc::smem_u32(smem + C::OFF_A + kb * A_BYTES));
+          const uint64_t b = tc::sdesc_sw128(tc::smem_u32(smem + C::OFF_B + kb * B_BYTES));
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            tc::mma_bf16(tmem, tc::sdesc_sw128(a + 32 * k), tc::sdesc_sw128(b + 32 * k), id64, (kb | k) ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) tc::mma_bf16(tmem, a + 2 * k, b + 2 * k, id64, (kb | k) ? 1u : 0u);
         }
         tc::mma_commit(done);
       }
@@ -1385,10 +1384,10 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
         if (*abort) continue;  // issue nothing after a timeout
         issued = true;
         tc::tc_fence_after();
-        const uint32_t a = tc::smem_u32(smem + C::OFF_A + q * A_BYTES), b = tc::smem_u32(smem + C::OFF_B + q * B_BYTES);
+        const uint64_t a = tc::sdesc_sw128(tc::smem_u32(smem + C::OFF_A + q * A_BYTES));
+        const uint64_t b = tc::sdesc_sw128(tc::smem_u32(smem + C::OFF_B + q * B_BYTES));
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          tc::mma_bf16(tmem, tc::sdesc_sw128(a + 32 * k), tc::sdesc_sw128(b + 32 * k), id64, (kb | k) ? 1u : 0u);
+        for (int k = 0; k < 4; ++k) tc::mma_bf16(tmem, a + 2 * k, b + 2 * k, id64, (kb | k) ? 1u : 0u);
         tc::mma_commit(&empty[q]);
       }
       if (!*abort) tc::mma_commit(done);
