@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
     if (!*abort) tc::mma_commit(done);
   }
 
-  if (warp < 4 && !fwd_epilogue(smem, OFF_A, OFF_W1, OFF_W2, tmem, done, 0, r, live, c, cols, h1g, h2g, og,
+  if (warp < 8 && !fwd_epilogue<2>(smem, OFF_A, OFF_W1, OFF_W2, tmem, done, 0, r, live, c, cols, h1g, h2g, og,
                                   write_hidden, sa, abort, limit, &issued, w1s, w1bar))
     ok = false;
   tc::tc_fence_before();
@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(TmaCfg::THREADS, 1)
         tc::mbar_arrive(&afull[a]);
       }
       const int c = c0 + tile * TILE + r;
-      if (!fwd_epilogue(smem, C::OFF_A, C::OFF_W1, C::OFF_W2, tmem, done, 3 * t, r, c < c1, c, cols, h1g, h2g, og,
+      if (!fwd_epilogue<1>(smem, C::OFF_A, C::OFF_W1, C::OFF_W2, tmem, done, 3 * t, r, c < c1, c, cols, h1g, h2g, og,
                         write_hidden, sa, abort, limit, &issued))
         ok = false;
     }

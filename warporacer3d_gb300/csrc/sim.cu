@@ -1229,7 +1229,8 @@ __global__ void k_lidar_spot(TrackDev t, int max_iters, const float4* __restrict
 // its place in the next step's A operand, so that the forward loads nothing.
 // Wider inputs take their k-blocks through the stages, a row in parts by
 // several threads. 100 steps of 1024 cars x 108 beams: 2.03 ms against 2.32 with
-// a thread a row and four round trips to L2 for each k-block.
+// a thread a row and four round trips to L2 for each k-block (before the
+// epilogue's rows were shared by two threads).
 // Data the kernel rewrites every step (obs, the ray frames, actions) is read
 // with coherent loads (never the read-only path); the block's barrier orders
 // its writes before the next phase's reads.
@@ -1392,10 +1393,10 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
       }
       if (!*abort) tc::mma_commit(done);
     }
-    if (warp < 4) {
+    if (warp < 8) {
       SampleArgs sk = sa;
       sk.step_add = sa.step_add + step;
-      if (!fwd_epilogue(smem, C::OFF_A, C::OFF_W1, C::OFF_W2, tmem, done, 3u * (uint32_t)step, r, live, c, n, nullptr,
+      if (!fwd_epilogue<2>(smem, C::OFF_A, C::OFF_W1, C::OFF_W2, tmem, done, 3u * (uint32_t)step, r, live, c, n, nullptr,
                         nullptr, og, 0, sk, abort, limit, &issued))
         ok = false;
     }
