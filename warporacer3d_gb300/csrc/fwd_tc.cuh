@@ -29,7 +29,8 @@ constexpr int B_BYTES = 64 * 128;    // 64 rows x 64 bf16
 // With w1s, W1 is not resident: thread 0 copies it to OFF_W1 once layer 1 is done (w1bar).
 // A row's 64 tanh and their packing stand in the way of the next layer, so two
 // groups share them where eight warps are at hand: 100 fused steps of 1024
-// cars take 1.81 ms against 2.00 with one.
+// cars take 1.81 ms against 2.00 with one (1.80 once warps without a row of
+// the batch skip theirs).
 template <int PARTS>
 __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, uint32_t tmem, uint64_t* done,
                              uint32_t p0, int r, bool live, int c, int cols, float* h1g, float* h2g, float* og,
@@ -51,32 +52,36 @@ __device__ bool fwd_epilogue(uint8_t* smem, int OFF_A, int OFF_W1, int OFF_W2, u
       tc::bulk_load(smem + OFF_W1, w1s, 2 * B_BYTES, w1bar);
     }
     float acc[UNITS];
+    const bool busy = __any_sync(0xffffffffu, live);  // a warp of rows past the batch has nothing to hand on
     for (int layer = 0; layer < 2; ++layer) {
-      if (!__any_sync(0xffffffffu, *abort != 0)) {  // warp-uniform: the loads are warp-collective
+      if (busy) {
+        if (!__any_sync(0xffffffffu, *abort != 0)) {  // warp-uniform: the loads are warp-collective
 #pragma unroll
-        for (int q = 0; q < UNITS / 16; ++q) tc::tmem_ld16(trow + UNITS * part + 16 * q, acc + 16 * q);
-        tc::tmem_wait_ld();
-      } else {
+          for (int q = 0; q < UNITS / 16; ++q) tc::tmem_ld16(trow + UNITS * part + 16 * q, acc + 16 * q);
+          tc::tmem_wait_ld();
+        } else {
 #pragma unroll
-        for (int q = 0; q < UNITS; ++q) acc[q] = 0.0f;
-      }
-#pragma unroll
-      for (int q = 0; q < UNITS; ++q) acc[q] = tc::tanh_fast(acc[q]);
-#pragma unroll
-      for (int q = 0; q < UNITS / 8; ++q) {
-        uint4 pk = make_uint4(tc::pack_bf16(acc[8 * q], acc[8 * q + 1]), tc::pack_bf16(acc[8 * q + 2], acc[8 * q + 3]),
-                              tc::pack_bf16(acc[8 * q + 4], acc[8 * q + 5]),
-                              tc::pack_bf16(acc[8 * q + 6], acc[8 * q + 7]));
-        *reinterpret_cast<uint4*>(Hs + r * 128 + (((UNITS / 8 * part + q) ^ (r & 7)) << 4)) = pk;
-        if (q < 2 && part == 0) {  // the bias's one and 15 zeros: the only step of 16 k's past h
-          const uint4 hi = make_uint4(q == 0 ? tc::pack_bf16(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
-          *reinterpret_cast<uint4*>(Hs + A_BYTES + r * 128 + ((q ^ (r & 7)) << 4)) = hi;
+          for (int q = 0; q < UNITS; ++q) acc[q] = 0.0f;
         }
-      }
-      if (write_hidden && live) {
-        float* hg = layer == 0 ? h1g : h2g;
 #pragma unroll
-        for (int q = 0; q < UNITS; ++q) hg[(long)(UNITS * part + q) * cols + c] = acc[q];
+        for (int q = 0; q < UNITS; ++q) acc[q] = tc::tanh_fast(acc[q]);
+#pragma unroll
+        for (int q = 0; q < UNITS / 8; ++q) {
+          uint4 pk = make_uint4(tc::pack_bf16(acc[8 * q], acc[8 * q + 1]),
+                                tc::pack_bf16(acc[8 * q + 2], acc[8 * q + 3]),
+                                tc::pack_bf16(acc[8 * q + 4], acc[8 * q + 5]),
+                                tc::pack_bf16(acc[8 * q + 6], acc[8 * q + 7]));
+          *reinterpret_cast<uint4*>(Hs + r * 128 + (((UNITS / 8 * part + q) ^ (r & 7)) << 4)) = pk;
+          if (q < 2 && part == 0) {  // the bias's one and 15 zeros: the only step of 16 k's past h
+            const uint4 hi = make_uint4(q == 0 ? tc::pack_bf16(1.0f, 0.0f) : 0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(Hs + A_BYTES + r * 128 + ((q ^ (r & 7)) << 4)) = hi;
+          }
+        }
+        if (write_hidden && live) {
+          float* hg = layer == 0 ? h1g : h2g;
+#pragma unroll
+          for (int q = 0; q < UNITS; ++q) hg[(long)(UNITS * part + q) * cols + c] = acc[q];
+        }
       }
       tc::fence_proxy_async_smem();
       tc::tc_fence_before();
