@@ -49,7 +49,7 @@ __device__ __forceinline__ int world_phase(float sh, float ch, int K, float* pha
 
 // World frame, inference: 16 world samples o0 .. o0 + 15 of one car (o0 a
 // multiple of 16, K of 16), saturated to [0, 1], rounded to FP16 into row
-// (16-byte aligned), and the smallest of those inside the car's field of view
+// (32-byte aligned: one store), and the smallest of those inside the car's field of view
 // (beam (o - k0) mod K < beams), taken before the rounding and rounded once
 // (rounding is monotonic, so that is the smallest rounded value). A group
 // with no sample in the field of view is not stored (nothing reads it). The

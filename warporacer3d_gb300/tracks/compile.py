@@ -101,7 +101,7 @@ def assemble(inp, grids, layers):
 def _compile(inp, run, what):
     """The packed array of `inp`, its grids written in place by the C ABI's `what` through `run`."""
     out = np.empty(HEADER + inp.grids_len() + 4 * len(inp.route), dtype=np.float32)
-    rc, _, layers = run(inp, getattr(_lib(), what), out[HEADER:HEADER + inp.grids_len()])
+    rc, layers = run(inp, getattr(_lib(), what), out[HEADER:HEADER + inp.grids_len()])[::2]
     _check(rc, what)
     head, tail = _ends(inp, layers)
     end = HEADER + layers * 3 * inp.nx * inp.ny
