@@ -1,5 +1,5 @@
-"""Where the lidar's launch changes with the size: warps across car boundaries once a car's last warp would leave more
-than a twelfth of the lanes idle, against the oracle; and a launch a segment in place of the segment table from 2^18
+"""Where the lidar's launch changes with the size: warps across car boundaries where a car's last warp would leave
+lanes idle, against the oracle; and a launch a segment in place of the segment table from 2^18
 blocks on, against the table (the same cars with more of them to a block), a segment of one car among them."""
 import numpy as np
 import pytest

@@ -1038,10 +1038,13 @@ template <int LAYERS, int CARS, bool WIDE>
 static void lidar_track(const TrackDev& t, int max_iters, const float4* ray, float* obs, int n, int c0, int c1,
                         int beams, const float2* beam_dir, int* iters, cudaStream_t st, bool flat, bool early) {
   const long items = (long)(c1 - c0) * beams;
-  // Warps across car boundaries where asked for, and where a car's last warp would leave more than a twelfth of the
-  // lanes idle: 108 beams (16%) at 16384 cars 58.0 us against 62.4; at 181 (6%) and 300 (6%) beams either takes as long.
+  // Warps across car boundaries where asked for, and where a car's last warp would idle some lanes: 108 beams (16% of
+  // them) at 16384 cars 58.0 us against 62.4, 271 (6%) at 2999 cars 27.1 us a step against 27.4, 1081 (0.6%) a 64-step
+  // rollout of 4096 cars 6.05 ms against 6.15. In grids of BIG_LIDAR blocks only above a twelfth: five tracks' 119,808
+  // cars at 1081 beams take 5.13 ms a step that way and 5.09 with a car's beams to themselves.
   const int lanes = (beams + 31) / 32 * 32;
-  if ((flat || (lanes - beams) * 12 > lanes) && items > 0 && items < (1L << 31)) {
+  const bool big = (long)((c1 - c0 + CARS - 1) / CARS) * (lanes / 32) >= BIG_LIDAR;
+  if ((flat || (big ? (lanes - beams) * 12 > lanes : lanes > beams)) && items > 0 && items < (1L << 31)) {
     const unsigned blocks = (unsigned)((items + 32 * CARS - 1) / (32 * CARS));
     lidar_launch(k_lidar_flat<LAYERS, CARS, WIDE>, dim3(blocks), CARS * 32, st, early, t, max_iters, ray, obs, n, c0,
                  (unsigned)items, beams, beam_dir, iters);
