@@ -109,7 +109,11 @@ inline int device_sms() {
 // Programmatic dependent launch: a kernel launched with `launch_early` becomes resident once every block of the kernel
 // before it in the stream has called early_next (or ended), and must call early_wait, which returns once that kernel
 // has completed, before it touches memory that another kernel does. Hides a launch's latency, and what a kernel sets up
-// for itself, behind its predecessor. Both calls do nothing in a kernel launched otherwise.
+// for itself, behind its predecessor. early_wait does nothing in a kernel launched otherwise; early_next releases
+// whatever early launch follows, however its own kernel was launched.
+// The kernels before it write while such a kernel is resident, so what any of them writes is read by plain, __ldcg or
+// __ldcs loads and not through the read-only path (__ldg, const __restrict__), which requires memory that stays as it
+// is and whose loads may move above early_wait. Tracks and beam tables, which no kernel writes, keep that path.
 __device__ __forceinline__ void early_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void early_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void early_start() {

@@ -63,11 +63,8 @@ struct FwdCfg {
 // epilogues and issue layers 2 and 3.
 template <int GROUPS>
 __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
-    k_mlp_fwd(const float* __restrict__ x, int in, int cols, int c0, int c1,
-                                                        const uint4* __restrict__ w0s, int kblocks,
-                                                        const uint4* __restrict__ w1s,
-                                                        const uint4* __restrict__ w2s, float* h1g, float* h2g,
-                                                        float* og, int write_hidden, SampleArgs sa, int* err) {
+    k_mlp_fwd(const float* x, int in, int cols, int c0, int c1, const uint4* w0s, int kblocks, const uint4* w1s,
+              const uint4* w2s, float* h1g, float* h2g, float* og, int write_hidden, SampleArgs sa, int* err) {
   using C = FwdCfg<GROUPS>;
   constexpr int THREADS = C::THREADS, MMA_WARP = C::MMA_WARP, OFF_A = C::OFF_A, OFF_B = C::OFF_B,
                 OFF_W1 = C::OFF_W1, OFF_W2 = C::OFF_W2, OFF_BAR = C::OFF_BAR;
@@ -107,7 +104,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
   early_wait();
   {  // W2 (2 x 2 KB), resident for the whole tile
     uint4* w2 = reinterpret_cast<uint4*>(smem + OFF_W2);
-    for (int e = tid; e < 2 * 16 * 128 / 16; e += THREADS) w2[e] = __ldg(w2s + e);
+    for (int e = tid; e < 2 * 16 * 128 / 16; e += THREADS) w2[e] = __ldcg(w2s + e);
   }
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();
@@ -130,12 +127,12 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
 #pragma unroll
       for (int q = 0; q < 64; ++q) {
         const int f = kb * 64 + q;
-        v[q] = (live && f < in) ? __ldg(x + (long)f * cols + c) : 0.0f;
+        v[q] = (live && f < in) ? __ldcg(x + (long)f * cols + c) : 0.0f;
       }
       uint4 wb[4];
       const uint4* src = w0s + (long)kb * (B_BYTES / 16);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) wb[e] = __ldg(src + r + e * TILE);
+      for (int e = 0; e < 4; ++e) wb[e] = __ldcg(src + r + e * TILE);
       if (j >= 1 && !tc::mbar_wait_abort(&empty[g], (j - 1) & 1, abort, limit)) ok = false;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
@@ -217,9 +214,9 @@ static_assert(TmaCfg::SMEM_BYTES <= 227 * 1024, "one CTA per SM");
 static_assert((2 * XS + 2 * XA + 3) * 8 + 8 <= 256, "barriers, the TMEM slot and the abort word fit their 256 bytes");
 
 __global__ void __launch_bounds__(TmaCfg::THREADS, 1)
-    k_mlp_fwd_tma(const __grid_constant__ CUtensorMap xmap, int cols, int c0, int c1, const uint4* __restrict__ w0s,
-                  int kblocks, const uint4* __restrict__ w1s, const uint4* __restrict__ w2s, float* h1g, float* h2g,
-                  float* og, int write_hidden, SampleArgs sa, int* err) {
+    k_mlp_fwd_tma(const __grid_constant__ CUtensorMap xmap, int cols, int c0, int c1, const uint4* w0s, int kblocks,
+                  const uint4* w1s, const uint4* w2s, float* h1g, float* h2g, float* og, int write_hidden,
+                  SampleArgs sa, int* err) {
   using C = TmaCfg;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = tc::smem_u32(smem_raw);
@@ -262,8 +259,8 @@ __global__ void __launch_bounds__(TmaCfg::THREADS, 1)
   {  // W1 (2 x 8 KB) and W2 (2 x 2 KB), resident for the whole tile
     uint4* w1 = reinterpret_cast<uint4*>(smem + C::OFF_W1);
     uint4* w2 = reinterpret_cast<uint4*>(smem + C::OFF_W2);
-    for (int e = tid; e < 2 * B_BYTES / 16; e += C::THREADS) w1[e] = __ldg(w1s + e);
-    for (int e = tid; e < 2 * 16 * 128 / 16; e += C::THREADS) w2[e] = __ldg(w2s + e);
+    for (int e = tid; e < 2 * B_BYTES / 16; e += C::THREADS) w1[e] = __ldcg(w1s + e);
+    for (int e = tid; e < 2 * 16 * 128 / 16; e += C::THREADS) w2[e] = __ldcg(w2s + e);
   }
   tc::fence_proxy_async_smem();
   tc::tc_fence_before();

@@ -647,11 +647,11 @@ __global__ void k_rk4_f64(const __grid_constant__ Segments g, const float* prev,
 // 243-249): pose (x, y, heading, layer) -> z = the layer's bilinear height,
 // the slopes along and across the heading, and the same frame k_advance
 // writes. Used to label surrogate training poses with the exact tracer.
-__global__ void k_pose_frames(TrackDev t, const float4* __restrict__ poses, int count, float4* ray) {
+__global__ void k_pose_frames(TrackDev t, const float4* poses, int count, float4* ray) {
   early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const float4 p = poses[i];
+  const float4 p = __ldcg(poses + i);
   const int layer = (int)p.w;
   const Surface g = surface(t, layer, p.x, p.y);
   float along, across;
@@ -676,7 +676,7 @@ __global__ void k_pose_frames(TrackDev t, const float4* __restrict__ poses, int 
 // the probe count (dropped where its bound cannot end the march) and
 // floor/descent (quotient: two residual corrections of the reciprocal; the
 // guarded march divides only where min() can select it).
-template <int LAYERS, bool NC = true>
+template <int LAYERS>
 __device__ __forceinline__ void trace(const TrackDev& t, const float4* ray, float* obs, int n,
                                       const float2* __restrict__ beam_dir, int max_iters, int* iters, int car,
                                       int beam);
@@ -688,7 +688,7 @@ struct LidarGrid {
   int block0[MAX_SEGMENTS + 1];
 };
 
-__device__ __forceinline__ void trace_any(const TrackDev& t, const float4* __restrict__ ray, float* obs, int n,
+__device__ __forceinline__ void trace_any(const TrackDev& t, const float4* ray, float* obs, int n,
                                           const float2* __restrict__ beam_dir, int max_iters, int* iters, int car,
                                           int beam) {
   if (t.layers == 1)
@@ -710,7 +710,7 @@ constexpr int lidar_min_blocks(int cars, bool wide) {
 // blocks release their slot as soon as their few cars finish.
 template <int LAYERS, int CARS, bool WIDE>
 __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
-    k_lidar_track(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0, int c1,
+    k_lidar_track(TrackDev t, int max_iters, const float4* ray, float* obs, int n, int c0, int c1,
                   int beams, const float2* __restrict__ beam_dir, int* iters) {
   early_start();
   const int beam = blockIdx.y * 32 + (threadIdx.x & 31);
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
 // 3.375 warps a car). Each beam is traced exactly as in k_lidar_track.
 template <int LAYERS, int CARS, bool WIDE>
 __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
-    k_lidar_flat(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0,
+    k_lidar_flat(TrackDev t, int max_iters, const float4* ray, float* obs, int n, int c0,
                  unsigned items, int beams, const float2* __restrict__ beam_dir, int* iters) {
   early_start();
   const unsigned item = (blockIdx.x * CARS + (threadIdx.x >> 5)) * 32u + (threadIdx.x & 31);
@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
 // no tail of idle slots.
 template <int LAYERS, bool WIDE>
 __global__ void __launch_bounds__(128, lidar_min_blocks(4, WIDE))
-    k_lidar_dynamic(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int c0, int c1,
+    k_lidar_dynamic(TrackDev t, int max_iters, const float4* ray, float* obs, int n, int c0, int c1,
                     int beams, const float2* __restrict__ beam_dir, int* iters, unsigned* counter) {
   const int groups = (beams + 31) >> 5;
   const unsigned total = (unsigned)(c1 - c0) * (unsigned)groups;
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(128, lidar_min_blocks(4, WIDE))
 // units from a counter took 104, 64 that claim them 108.
 template <int LAYERS>
 __global__ void __launch_bounds__(128, lidar_min_blocks(4, false))
-    k_lidar_list(TrackDev t, int max_iters, const float4* __restrict__ ray, float* obs, int n, int beams,
+    k_lidar_list(TrackDev t, int max_iters, const float4* ray, float* obs, int n, int beams,
                  const float2* __restrict__ beam_dir, const int* __restrict__ list, const int* list_count) {
   const unsigned groups = (unsigned)(beams + 31) >> 5, total = (unsigned)min(max(*list_count, 0), n) * groups;
   const unsigned warps = gridDim.x * (blockDim.x >> 5);
@@ -783,8 +783,8 @@ __global__ void __launch_bounds__(128, lidar_min_blocks(4, false))
 template <int CARS, bool WIDE>
 __global__ void __launch_bounds__(CARS * 32, lidar_min_blocks(CARS, WIDE))
     k_lidar_segments(const __grid_constant__ Segments g, const __grid_constant__ LidarGrid lg,
-                     const float4* __restrict__ ray, float* obs, int n, int beams,
-                     const float2* __restrict__ beam_dir, int* iters) {
+                     const float4* ray, float* obs, int n, int beams, const float2* __restrict__ beam_dir,
+                     int* iters) {
   early_start();
   const int beam = blockIdx.y * 32 + (threadIdx.x & 31);
   if (beam >= beams) return;
@@ -800,10 +800,10 @@ __device__ __forceinline__ float march(const TrackDev& t, float ox, float oy, fl
                                        float descent, float inv_descent, int max_iters, int* count_out);
 
 // The range of one beam (racer/sim.mojo:240-266); `count` gets its probes.
-// NC: the ray frames are read-only for the whole launch (the read-only data
-// path); the fused rollout, which rewrites them every step, loads them
-// through L2 instead, where the block's own writes before a barrier are seen.
-template <int LAYERS, bool NC = true>
+// The ray frames are loaded through L2, never by the read-only path: a lidar
+// launched early is resident while the kernel before it still writes them, and
+// the fused rollout rewrites them every step.
+template <int LAYERS>
 __device__ __forceinline__ float beam_range(const TrackDev& t, const float4* ray, int n,
                                             const float2* __restrict__ beam_dir, int max_iters, bool counted,
                                             int car, int beam, int* count_out);
@@ -822,22 +822,22 @@ __device__ __forceinline__ float range_obs(float range) {
   return range < 8.67361738e-19f ? range / RANGE : quotient(range, RANGE, 0.1f, range * 0.1f);
 }
 
-template <int LAYERS, bool NC>
+template <int LAYERS>
 __device__ __forceinline__ void trace(const TrackDev& t, const float4* ray, float* obs, int n,
                                       const float2* __restrict__ beam_dir, int max_iters, int* iters, int car,
                                       int beam) {
   int count = 0;
-  const float range = beam_range<LAYERS, NC>(t, ray, n, beam_dir, max_iters, iters != nullptr, car, beam, &count);
+  const float range = beam_range<LAYERS>(t, ray, n, beam_dir, max_iters, iters != nullptr, car, beam, &count);
   obs[(long)(4 + beam) * n + car] = range_obs(range);
   if (iters) iters[(long)beam * n + car] = count;
 }
 
-template <int LAYERS, bool NC>
+template <int LAYERS>
 __device__ __forceinline__ float beam_range(const TrackDev& t, const float4* ray, int n,
                                             const float2* __restrict__ beam_dir, int max_iters, bool counted,
                                             int car, int beam, int* count_out) {
   // (ox, oy, oz, cos h), (sin h, along, across)
-  const float4 r0 = NC ? __ldg(ray + car) : __ldcg(ray + car), r1 = NC ? __ldg(ray + n + car) : __ldcg(ray + n + car);
+  const float4 r0 = __ldcg(ray + car), r1 = __ldcg(ray + n + car);
   const float2 az = __ldg(beam_dir + beam);                        // (cos azimuth, sin azimuth)
   float dx = az.x * r0.w + az.y * -r1.x;
   float dy = az.x * r1.x + az.y * r0.w;
@@ -1416,11 +1416,11 @@ __global__ void __launch_bounds__(FusedRolloutCfg::THREADS, 2)
       if (beam >= beams) continue;
       if (RESIDENT) {
         int count;
-        const float v = range_obs(beam_range<LAYERS, false>(t, ray, n, beam_dir, g.max_iters[0], false, car, beam, &count));
+        const float v = range_obs(beam_range<LAYERS>(t, ray, n, beam_dir, g.max_iters[0], false, car, beam, &count));
         obs[(long)(4 + beam) * n + car] = v;
         *fused_input(smem + C::OFF_A, car - c0, 4 + beam) = __float2bfloat16_rn(v);
       } else {
-        trace<LAYERS, false>(t, ray, obs, n, beam_dir, g.max_iters[0], nullptr, car, beam);
+        trace<LAYERS>(t, ray, obs, n, beam_dir, g.max_iters[0], nullptr, car, beam);
       }
     }
     if (RESIDENT) {  // the other inputs, and zeros to the k-block's end, where the forward left its activations

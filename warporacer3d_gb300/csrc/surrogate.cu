@@ -152,12 +152,12 @@ __device__ __forceinline__ void load_bias(const float* bias, int n, int N, float
   if (n + 16 <= N) {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float4 f = __ldg(reinterpret_cast<const float4*>(bias + n) + q);
+      const float4 f = *(reinterpret_cast<const float4*>(bias + n) + q);
       out[4 * q] = f.x, out[4 * q + 1] = f.y, out[4 * q + 2] = f.z, out[4 * q + 3] = f.w;
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < 16; ++j) out[j] = n + j < N ? __ldg(bias + n + j) : 0.0f;
+    for (int j = 0; j < 16; ++j) out[j] = n + j < N ? bias[n + j] : 0.0f;
   }
 }
 
@@ -227,11 +227,11 @@ struct EpiLoss {
     int first = 0;
     if (WORLD) {
       if (n >= ldgs) return;  // n is a multiple of 16, ldgs of 64
-      first = row ? __ldg(k0 + m) : 0;
+      first = row ? __ldcg(k0 + m) : 0;
       const float4* src = reinterpret_cast<const float4*>(target + (long)m * ldgs + n);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float4 f = row ? __ldg(src + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const float4 f = row ? src[q] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);  // half a sector: L1 has the rest
         t[4 * q] = f.x, t[4 * q + 1] = f.y, t[4 * q + 2] = f.z, t[4 * q + 3] = f.w;
       }
     }
@@ -367,18 +367,18 @@ __device__ __forceinline__ void store_inputs(const float* f, int i, bf16* x) {
   for (int q = 0; q < NIN / 16; ++q) store16(x + (long)i * NIN + 16 * q, f + 16 * q);
 }
 
-__global__ void k_features(const float4* __restrict__ ray, int count, Norm nm, bf16* x) {
+__global__ void k_features(const float4* ray, int count, Norm nm, bf16* x) {
   early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const float4 r0 = ray[i], r1 = ray[count + i];
+  const float4 r0 = __ldcg(ray + i), r1 = __ldcg(ray + count + i);
   float f[NIN];
   encode((r0.x - nm.xc) * nm.inv_xs, (r0.y - nm.yc) * nm.inv_ys, r0.z, r1.x, r0.w, r1.w, f);
   store_inputs(f, i, x);
 }
 
 // The feature grids of `layer` at (ox, oy), level by level, into f[0 .. 39].
-__device__ __forceinline__ void grid_features(const GridGeom& gg, const float* __restrict__ grid, float ox, float oy,
+__device__ __forceinline__ void grid_features(const GridGeom& gg, const float* grid, float ox, float oy,
                                               int layer, float* f) {
 #pragma unroll
   for (int l = 0; l < GRID_LEVELS; ++l) {
@@ -388,10 +388,10 @@ __device__ __forceinline__ void grid_features(const GridGeom& gg, const float* _
     const float w00 = (1.0f - fu) * (1.0f - fv), w10 = fu * (1.0f - fv), w01 = (1.0f - fu) * fv, w11 = fu * fv;
 #pragma unroll
     for (int q = 0; q < GRID_F / 4; ++q) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(grid + c) + q);
-      const float4 b = __ldg(reinterpret_cast<const float4*>(grid + c + GRID_F) + q);
-      const float4 d = __ldg(reinterpret_cast<const float4*>(grid + c + dy) + q);
-      const float4 e = __ldg(reinterpret_cast<const float4*>(grid + c + dy + GRID_F) + q);
+      const float4 a = *(reinterpret_cast<const float4*>(grid + c) + q);
+      const float4 b = *(reinterpret_cast<const float4*>(grid + c + GRID_F) + q);
+      const float4 d = *(reinterpret_cast<const float4*>(grid + c + dy) + q);
+      const float4 e = *(reinterpret_cast<const float4*>(grid + c + dy + GRID_F) + q);
       float* o = f + GRID_F * l + 4 * q;
       o[0] = w00 * a.x + w10 * b.x + w01 * d.x + w11 * e.x;
       o[1] = w00 * a.y + w10 * b.y + w01 * d.y + w11 * e.y;
@@ -406,12 +406,12 @@ __device__ __forceinline__ void grid_features(const GridGeom& gg, const float* _
 //   40..47  x', y', z, sin h, cos h, [layer 0], [layer 1], 1
 //   48..55  sin/cos(j h) for j = 2..5
 //   56..63  sin/cos(2^k pi x'), sin/cos(2^k pi y') for k = 0, 1
-__global__ void k_features_cargrid(const float4* __restrict__ ray, int count, Norm nm, GridGeom gg,
-                                   const float* __restrict__ grid, bf16* x) {
+__global__ void k_features_cargrid(const float4* ray, int count, Norm nm, GridGeom gg, const float* grid,
+                                   bf16* x) {
   early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const float4 r0 = ray[i], r1 = ray[count + i];
+  const float4 r0 = __ldcg(ray + i), r1 = __ldcg(ray + count + i);
   const int layer = r1.w == 1.0f ? 1 : 0;
   float f[NIN];
   grid_features(gg, grid, r0.x, r0.y, layer, f);
@@ -439,12 +439,12 @@ __global__ void k_features_cargrid(const float4* __restrict__ ray, int count, No
 //   40..45  x', y', z, [layer 0], [layer 1], 1
 //   46..61  sin/cos(2^k pi x'), sin/cos(2^k pi y') for k = 0..3
 //   62, 63  sin/cos(2 pi phase)
-__global__ void k_features_world(const float4* __restrict__ ray, int count, Norm nm, GridGeom gg,
-                                 const float* __restrict__ grid, int K, bf16* x) {
+__global__ void k_features_world(const float4* ray, int count, Norm nm, GridGeom gg, const float* grid, int K,
+                                 bf16* x) {
   early_start();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
-  const float4 r0 = ray[i], r1 = ray[count + i];
+  const float4 r0 = __ldcg(ray + i), r1 = __ldcg(ray + count + i);
   const int layer = r1.w == 1.0f ? 1 : 0;
   float f[NIN];
   grid_features(gg, grid, r0.x, r0.y, layer, f);
@@ -471,8 +471,8 @@ __global__ void k_features_world(const float4* __restrict__ ray, int count, Norm
 // World frame, training: every sample's labels at the world samples its beams read, rows[m * ld + (k0 + b) mod K] =
 // target[b * B + m], and k0. A block turns 32 samples x 32 beams over in shared memory: 128-byte rows in, runs of 32
 // world samples out (the loss epilogue reads whole rows; reading the labels from there took a 32-byte sector a value).
-__global__ void __launch_bounds__(256) k_world_targets(const float* __restrict__ target, const float4* __restrict__ ray,
-                                                       int B, int beams, int K, int ld, float* rows, int* k0) {
+__global__ void __launch_bounds__(256) k_world_targets(const float* target, const float4* ray, int B, int beams, int K,
+                                                       int ld, float* rows, int* k0) {
   early_start();
   __shared__ float tile[32][33];
   __shared__ int first[32];
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(256) k_world_targets(const float* __restrict__
   if (row == 0) {
     float ph;
     const int m = m0 + lane;
-    first[lane] = m < B ? world_phase(ray[B + m].x, ray[m].w, K, &ph) : 0;
+    first[lane] = m < B ? world_phase(__ldcg(ray + B + m).x, __ldcg(ray + m).w, K, &ph) : 0;
     if (blockIdx.y == 0 && m < B) k0[m] = first[lane];
   }
 #pragma unroll
@@ -500,12 +500,11 @@ __global__ void __launch_bounds__(256) k_world_targets(const float* __restrict__
 // World frame: gradient of the feature grids from dL/df (dx [B, 64], FP32):
 // each sample's bilinear weights scatter its first 40 input gradients onto the
 // four corners of its cell at every level (16-byte atomic adds).
-__global__ void k_grid_grad(const float4* __restrict__ ray, int B, GridGeom gg, const float* __restrict__ dx,
-                            float* ggrad) {
+__global__ void k_grid_grad(const float4* ray, int B, GridGeom gg, const float* dx, float* ggrad) {
   early_start();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= B) return;
-  const float4 r0 = ray[m], r1 = ray[B + m];
+  const float4 r0 = __ldcg(ray + m), r1 = __ldcg(ray + B + m);
   const int layer = r1.w == 1.0f ? 1 : 0;
 #pragma unroll
   for (int l = 0; l < GRID_LEVELS; ++l) {
@@ -612,7 +611,7 @@ __global__ void k_sample_poses(const int2* cells, int ncells, int count, uint64_
 }
 
 // Sum of split-K partials into a row-major gradient block of `count` floats (a multiple of 4), four per thread.
-__global__ void k_reduce_splits(const float* __restrict__ P, int splits, long mn, long count, float* out) {
+__global__ void k_reduce_splits(const float* P, int splits, long mn, long count, float* out) {
   early_start();
   const long e = 4 * ((long)blockIdx.x * blockDim.x + threadIdx.x);
   if (e >= count) return;

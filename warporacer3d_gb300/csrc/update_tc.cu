@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
   {
     auto copy = [&](int off, const uint8_t* src, int bytes) {
       const uint4* s = reinterpret_cast<const uint4*>(src);
-      for (int e = tid; e < bytes / 16; e += C::THREADS) reinterpret_cast<uint4*>(smem + off)[e] = __ldg(s + e);
+      for (int e = tid; e < bytes / 16; e += C::THREADS) reinterpret_cast<uint4*>(smem + off)[e] = __ldcg(s + e);
     };
     const int w0_bytes = (in + 63) / 64 * W_BYTES;
     for (int e = tid; e < TILE_BYTES / 16; e += C::THREADS)  // unit 0 of every sample is 1
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
     copy(C::W1T, a.w1t, W_BYTES);
     if (tid < H) {
       const float* w = a.theta + w2 + tid;
-      w2f[tid] = make_float4(__ldg(w), __ldg(w + HA), __ldg(w + 2 * HA), 0.0f);
+      w2f[tid] = make_float4(__ldcg(w), __ldcg(w + HA), __ldcg(w + 2 * HA), 0.0f);
     }
   }
   tc::fence_proxy_async_smem();
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
   float ls[2], invvar[2], adv_mean, adv_scale;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
-    ls[k] = __ldg(a.theta + logstd + k);
+    ls[k] = __ldcg(a.theta + logstd + k);
     invvar[k] = rmath::expf_(-2.0f * ls[k]);
   }
   advantage_moments(a.moments, batch, &adv_mean, &adv_scale);
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
     }
     float s[5];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) s[k] = live ? __ldg(a.samples + (long)k * batch + j) : 0.0f;
+    for (int k = 0; k < 5; ++k) s[k] = live ? __ldcg(a.samples + (long)k * batch + j) : 0.0f;
 
     float h1[UNITS], v[UNITS];
     read(0, h1);  // (the last tile's products, its weight gradients among them, were issued before and are done too)
@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(UpdateCfg::THREADS, 1)
 // squares[block] = the block's sum of grad^2. The last block takes the log-std
 // gradients and the KL from the CTAs' sums.
 constexpr int RED_W = 32;
-__global__ void __launch_bounds__(RED_W * 32) k_update_reduce(const float* __restrict__ part, int ranges,
-                                                             const double* __restrict__ sums, int ctas, int weights,
-                                                             float* grad, double* squares, float* stats) {
+__global__ void __launch_bounds__(RED_W * 32) k_update_reduce(const float* part, int ranges, const double* sums,
+                                                             int ctas, int weights, float* grad, double* squares,
+                                                             float* stats) {
   __shared__ float sh[32][RED_W + 1];
   __shared__ double sq[32];
   early_start();
@@ -431,7 +431,7 @@ __global__ void __launch_bounds__(RED_W * 32) k_update_reduce(const float* __res
     float acc = 0.0f;
     if (p < weights)
 #pragma unroll 5
-      for (int z = row; z < ranges; z += 32) acc += part[(long)z * weights + p];
+      for (int z = row; z < ranges; z += 32) acc += __ldcg(part + (long)z * weights + p);
     sh[row][lane] = acc;
     __syncthreads();
     g = sh[lane][row];  // now weight `row` of the block, slice `lane`
@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(RED_W * 32) k_update_reduce(const float* __res
   if (row) return;
   double s[3] = {0.0, 0.0, 0.0};
   for (int c = lane; c < ctas; c += 32)
-    for (int k = 0; k < 3; ++k) s[k] += sums[c * 3 + k];
+    for (int k = 0; k < 3; ++k) s[k] += __ldcg(sums + c * 3 + k);
 #pragma unroll
   for (int k = 0; k < 3; ++k)
     for (int o = 16; o; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
@@ -465,14 +465,13 @@ __global__ void __launch_bounds__(RED_W * 32) k_update_reduce(const float* __res
 // racer/ppo.mojo:306-337: the gradient's norm (every block adds the partial
 // sums in the same order), Adam, and the new theta's BF16 operand images
 // (layouts of k_pack_weights and k_pack_w1t).
-__global__ void __launch_bounds__(256) k_update_adam(int in, int parts, const double* __restrict__ squares,
-                                                     const float* c12, float* stats, float* theta,
-                                                     const float* __restrict__ grad, float* first, float* second,
-                                                     uint8_t* pack, bf16* w1t) {
+__global__ void __launch_bounds__(256) k_update_adam(int in, int parts, const double* squares, const float* c12,
+                                                     float* stats, float* theta, const float* grad, float* first,
+                                                     float* second, uint8_t* pack, bf16* w1t) {
   __shared__ double sh[256];
   early_start();
   double q = 0.0;
-  for (int k = threadIdx.x; k < parts; k += 256) q += squares[k];
+  for (int k = threadIdx.x; k < parts; k += 256) q += __ldcg(squares + k);
   sh[threadIdx.x] = q;
   __syncthreads();
   for (int s = 128; s > 0; s >>= 1) {
@@ -486,7 +485,7 @@ __global__ void __launch_bounds__(256) k_update_adam(int in, int parts, const do
   if (i >= logstd + 2) return;
   const float c1 = c12[0], c2 = c12[1];
   float scale = fminf(1.0f, MAX_NORM / (sqrtf(norm) + 1e-8f));
-  float g = grad[i] * scale;
+  float g = __ldcg(grad + i) * scale;
   float m = 0.9f * first[i] + 0.1f * g;
   float v = 0.999f * second[i] + (0.001f * g) * g;
   first[i] = m;
