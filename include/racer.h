@@ -81,8 +81,10 @@ int racer_sim_create_segments(int count, const float* const* tracks, const size_
  * group of cars (cars_per_block is then unused). flat (one-track sims and
  * split launches, not dynamic): 1 = each warp takes the next 32 (car, beam)
  * pairs in car-major order, across car boundaries, so no lane idles when the
- * beam count is not a multiple of 32. Setting a different shape drops the
- * sim's captured rollout graphs. */
+ * beam count is not a multiple of 32; 0 = a car's beams in warps of their own.
+ * A sim whose shape was neither set nor tuned takes the one that a rule on its
+ * cars and beams prefers, which racer_sim_get_lidar_shape then returns. Setting
+ * a different shape drops the sim's captured rollout graphs. */
 typedef struct {
   int cars_per_block;
   int wide;

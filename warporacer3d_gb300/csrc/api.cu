@@ -1467,7 +1467,7 @@ static void to_api(const racer_sim* s, const LidarShape& shape, racer_lidar_shap
   out->wide = shape.wide;
   out->split = shape.split;
   out->dynamic = shape.dynamic;
-  out->flat = shape.flat;
+  out->flat = s->seg.count == 1 && !shape.dynamic ? lidar_flat(shape, s->n, s->beams) : shape.flat == 1;
   int order[MAX_SEGMENTS];
   segment_order(s, shape, order);
   for (int j = 0; j < MAX_SEGMENTS; ++j) out->order[j] = j < s->seg.count ? order[j] : -1;

@@ -1034,17 +1034,23 @@ static void lidar_launch(void (*k)(P...), dim3 grid, unsigned threads, cudaStrea
   cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
+// The caller's choice where there is one (racer_sim_set_lidar_shape, the autotuner); else warps across car boundaries
+// where a car's last warp would idle some lanes: 108 beams (16% of them) at 16384 cars 58.0 us against 62.4, 271 (6%) at
+// 2999 cars 27.1 us a step against 27.4, 1081 (0.6%) a 64-step rollout of 4096 cars 6.05 ms against 6.15. In grids of
+// BIG_LIDAR blocks only above a twelfth: five tracks' 119,808 cars at 1081 beams take 5.13 ms a step that way and 5.09
+// with a car's beams to themselves.
+bool lidar_flat(const LidarShape& shape, long cars, int beams) {
+  if (shape.flat != FLAT_RULE) return shape.flat == 1;
+  const int lanes = (beams + 31) / 32 * 32;
+  const bool big = (cars + shape.cars - 1) / shape.cars * (lanes / 32) >= BIG_LIDAR;
+  return big ? (lanes - beams) * 12 > lanes : lanes > beams;
+}
+
 template <int LAYERS, int CARS, bool WIDE>
 static void lidar_track(const TrackDev& t, int max_iters, const float4* ray, float* obs, int n, int c0, int c1,
                         int beams, const float2* beam_dir, int* iters, cudaStream_t st, bool flat, bool early) {
   const long items = (long)(c1 - c0) * beams;
-  // Warps across car boundaries where asked for, and where a car's last warp would idle some lanes: 108 beams (16% of
-  // them) at 16384 cars 58.0 us against 62.4, 271 (6%) at 2999 cars 27.1 us a step against 27.4, 1081 (0.6%) a 64-step
-  // rollout of 4096 cars 6.05 ms against 6.15. In grids of BIG_LIDAR blocks only above a twelfth: five tracks' 119,808
-  // cars at 1081 beams take 5.13 ms a step that way and 5.09 with a car's beams to themselves.
-  const int lanes = (beams + 31) / 32 * 32;
-  const bool big = (long)((c1 - c0 + CARS - 1) / CARS) * (lanes / 32) >= BIG_LIDAR;
-  if ((flat || (big ? (lanes - beams) * 12 > lanes : lanes > beams)) && items > 0 && items < (1L << 31)) {
+  if (flat && items > 0 && items < (1L << 31)) {
     const unsigned blocks = (unsigned)((items + 32 * CARS - 1) / (32 * CARS));
     lidar_launch(k_lidar_flat<LAYERS, CARS, WIDE>, dim3(blocks), CARS * 32, st, early, t, max_iters, ray, obs, n, c0,
                  (unsigned)items, beams, beam_dir, iters);
@@ -1084,7 +1090,7 @@ static void lidar_segment(const Segments& g, int k, const float4* ray, float* ob
       lidar_dynamic<0, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, counter, shape.sms, st);
     return;
   }
-  const bool flat = shape.flat == 1;
+  const bool flat = lidar_flat(shape, c1 - c0, beams);
   if (t.layers == 1)
     lidar_track<1, CARS, WIDE>(t, g.max_iters[k], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);
   else if (t.layers == 2)
@@ -1108,7 +1114,7 @@ static void lidar_shape(const Segments& g, const LidarShape& shape, const float4
   // against 502 and 2000 cars of 540 beams 93 us against 69.
   if ((long)grid.x * grid.y >= BIG_LIDAR) {
     LidarShape one = shape;
-    one.dynamic = 0;  // as the table's
+    one.dynamic = 0, one.flat = FLAT_RULE;  // neither applies to launches that are not split
     for (int j = 0; j < g.count; ++j)
       lidar_segment<CARS, WIDE>(g, lg.order[j], ray, obs, n, beams, beam_dir, iters, st, one, true);
     return;
@@ -1156,7 +1162,7 @@ void launch_lidar_cars(const Segments& g, const LidarShape& shape, int c0, int c
   if (g.count != 1 || c1 <= c0) return;
   const TrackDev& t = g.t[0];
   const bool wide = shape.wide == 1;
-  const bool flat = shape.flat == 1, early = false;  // one chain's waiting blocks would hold another's places
+  const bool flat = lidar_flat(shape, c1 - c0, beams), early = false;  // one chain's waiting blocks would hold another's places
 #define RACER_LIDAR_CARS(CARS, WIDE)                                                                         \
   if (t.layers == 1)                                                                                          \
     lidar_track<1, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);   \

@@ -167,7 +167,8 @@ class Sim:
         """Lidar launch shape: cars per block (2, 4, 8), the 40-register variant (wide), per-segment
         launches on parallel streams (split), the segments' order (default: index order), the
         persistent grid with dynamically assigned (car, beam group) units (dynamic) and warps taking
-        (car, beam) pairs across car boundaries (flat)."""
+        (car, beam) pairs across car boundaries (flat: 1) or one car's beams alone (0). A sim whose shape
+        is neither set nor tuned takes the one that a rule on its cars and beams prefers."""
         order = list(range(len(self.cars))) if order is None else list(order)
         shape = LidarShape(cars_per_block, wide, split, dynamic,
                            (ctypes.c_int * 8)(*(order + [-1] * (8 - len(order)))), flat)
