@@ -77,3 +77,26 @@ def test_other_values_are_refused(flat):
     sim = W.Sim(W.track("bank"), 4, 9)
     with pytest.raises(W.RacerError):
         sim.set_lidar_shape(2, flat=flat)
+
+
+def test_the_rule_without_a_choice():
+    """k_lidar_flat from 2^13 blocks of two cars' own warps on, where a car's last warp would idle lanes; a rollout's
+    chains go by the whole sim; launches of one segment of several keep a car's beams together."""
+    track = W.track("bank")
+    for cars, beams, flat in ((4094, 108, 0), (4095, 108, 1), (4096, 96, 0), (6000, 96, 0), (480, 1081, 0),
+                              (481, 1081, 1), (482, 1081, 1)):
+        sim = W.Sim(track, cars, 9, beams=beams)
+        assert sim.lidar_shape()["flat"] == flat
+        assert lidar_kernels(step_of(sim)) == {"k_lidar_flat" if flat else "k_lidar_track"}, (cars, beams)
+    run = W.Runner(track, 4096, beams=108)
+    run.sim.set_chains(4)
+    run.rollout(2)
+    run.synchronize()
+    assert lidar_kernels(lambda: (run.rollout(2), run.synchronize())) == {"k_lidar_flat"}
+
+
+def test_segments_keep_a_cars_beams_together():
+    tracks = [W.track(name) for name in ("flat", "bridge", "bank", "ramp")]
+    sim = W.Sim.segments(tracks, [1, 9000, 5423, 997], [1, 2, 3, 4], beams=1081)  # 7712 x 34 blocks: a launch a segment
+    assert sim.lidar_shape()["flat"] == 0
+    assert lidar_kernels(step_of(sim)) == {"k_lidar_track"}

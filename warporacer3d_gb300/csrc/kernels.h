@@ -33,7 +33,7 @@ void launch_lidar(const TrackDev& t, const float4* ray, float* obs, int n, int b
 void launch_lidar_list(const TrackDev& t, const float4* ray, float* obs, int n, int beams, const float2* beam_dir,
                        const int* list, const int* list_count, int list_max, int sms, cudaStream_t st);
 bool lidar_shape_ok(const LidarShape& shape);  // a caller's choice: flat 0 or 1
-// Whether a one-track launch over `cars` cars runs k_lidar_flat under `shape`.
+// Whether a one-track sim of `cars` cars runs k_lidar_flat under `shape`.
 bool lidar_flat(const LidarShape& shape, long cars, int beams);
 // Spot check: beams (step % stride) + k stride of every car traced exactly and compared with the
 // predicted rows pred [beams, n]; cars off by more than tol (range / RANGE units) get minr = 0.

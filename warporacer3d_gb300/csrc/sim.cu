@@ -1035,15 +1035,22 @@ static void lidar_launch(void (*k)(P...), dim3 grid, unsigned threads, cudaStrea
 }
 
 // The caller's choice where there is one (racer_sim_set_lidar_shape, the autotuner); else warps across car boundaries
-// where a car's last warp would idle some lanes: 108 beams (16% of them) at 16384 cars 58.0 us against 62.4, 271 (6%) at
-// 2999 cars 27.1 us a step against 27.4, 1081 (0.6%) a 64-step rollout of 4096 cars 6.05 ms against 6.15. In grids of
-// BIG_LIDAR blocks only above a twelfth: five tracks' 119,808 cars at 1081 beams take 5.13 ms a step that way and 5.09
-// with a car's beams to themselves.
+// where a car's last warp would idle some lanes, in sims of at least FLAT_MIN blocks of a car's own warps. A step that
+// way as a fraction of one with a car's beams to themselves, alone on the GPU, on bridge / bank / flat / occupancy:
+//   108 beams (16% idle):   1000 cars 1.01 / 1.00 / 1.00 / 1.01, 16384 cars 0.97 / 0.96 / 0.98 / 1.03
+//   271 beams (6%):         1000 cars 0.99 / 1.00 / 1.00 / 1.01, 16384 cars 0.99 / 0.98 / 1.00 / 1.02
+//   1081 beams (0.6%):      1000 cars 0.99 / 0.99 / 1.01 / 1.00, 16384 cars 0.98 / 0.99 / 0.96 / 1.00
+// Below FLAT_MIN neither gains (the lidar alone is up to 4% slower across cars: 14.1 us against 13.4 at 16 cars of 108
+// beams on bank); from there on the built-in tracks do, also among passes of other sims (2999 cars x 271 beams: 30.5 us a
+// step against 31.4 on bridge, 28.8 against 28.2 on flat), while the occupancy map's long marches lose up to 4%. A rollout's
+// chains count as one: 16 of 256 cars x 1081 beams take 6.06 ms against 6.15. Launches of one segment of several keep a
+// car's beams together: 119,808 cars on five tracks take 4.96 ms a step at 1081 beams against 5.16 and 1.63 at 271 against
+// 1.82, 16,773 cars at 1081 beams 783 us against 841.
+constexpr long FLAT_MIN = 1 << 13;
 bool lidar_flat(const LidarShape& shape, long cars, int beams) {
   if (shape.flat != FLAT_RULE) return shape.flat == 1;
-  const int lanes = (beams + 31) / 32 * 32;
-  const bool big = (cars + shape.cars - 1) / shape.cars * (lanes / 32) >= BIG_LIDAR;
-  return big ? (lanes - beams) * 12 > lanes : lanes > beams;
+  const int warps = (beams + 31) / 32;
+  return 32 * warps > beams && (cars + shape.cars - 1) / shape.cars * warps >= FLAT_MIN;
 }
 
 template <int LAYERS, int CARS, bool WIDE>
@@ -1114,7 +1121,7 @@ static void lidar_shape(const Segments& g, const LidarShape& shape, const float4
   // against 502 and 2000 cars of 540 beams 93 us against 69.
   if ((long)grid.x * grid.y >= BIG_LIDAR) {
     LidarShape one = shape;
-    one.dynamic = 0, one.flat = FLAT_RULE;  // neither applies to launches that are not split
+    one.dynamic = 0, one.flat = 0;  // neither applies to launches that are not split
     for (int j = 0; j < g.count; ++j)
       lidar_segment<CARS, WIDE>(g, lg.order[j], ray, obs, n, beams, beam_dir, iters, st, one, true);
     return;
@@ -1162,7 +1169,7 @@ void launch_lidar_cars(const Segments& g, const LidarShape& shape, int c0, int c
   if (g.count != 1 || c1 <= c0) return;
   const TrackDev& t = g.t[0];
   const bool wide = shape.wide == 1;
-  const bool flat = lidar_flat(shape, c1 - c0, beams), early = false;  // one chain's waiting blocks would hold another's places
+  const bool flat = lidar_flat(shape, n, beams), early = false;  // one chain's waiting blocks would hold another's places
 #define RACER_LIDAR_CARS(CARS, WIDE)                                                                         \
   if (t.layers == 1)                                                                                          \
     lidar_track<1, CARS, WIDE>(t, g.max_iters[0], ray, obs, n, c0, c1, beams, beam_dir, iters, st, flat, early);   \
