@@ -6,7 +6,7 @@
 //   layer 2  D[128, 64]  = [h1 | 1][128, 128] . W1^T (K = 65 padded to 128)
 //   layer 3  D[128, 16]  = [h2 | 1][128, 128] . W2^T (N = 3 padded to 16)
 //
-// X arrives feature-major FP32 [IN, cols] (the reference's layout); the CTA's
+// X arrives feature-major FP32 [IN, cols] (the reference's layout); groups of
 // four warps load it coalesced along the samples, convert to BF16 and store
 // the transposed K-major tile into 128B-swizzled shared memory (two stages,
 // overlapped with the MMAs of the previous k-block). W0 k-blocks and the
@@ -30,37 +30,44 @@
 namespace racer {
 namespace {
 
-// Two producer groups of four warps, one k-block in flight each in registers
-// (64 KB of loads an SM, 128 KB with two CTAs), plus one MMA warp; four groups
-// for wide inputs of a few samples, where only a CTA's own latency counts. Shared
-// memory is kept to 54 KB: the SM's L1 is what its resident CTAs leave of 256
-// KB, and the lidar of another rollout chain or stream that shares the SM
-// gathers its cells through it (k_lidar_track at 4096 cars x 1081 beams takes
-// 119 us with 224 KB of L1, 122 with 118 KB, 133 with 28 KB). So W1 takes the
-// place of W0's stages once layer 1 is done (a bulk copy behind the first
-// tanh), and no stage is deeper than the loads in flight need. The TMA-staged
-// kernel below (200 KB) in this place made a 64-step rollout of 4096 cars in
-// 16 chains 7.12 ms against 6.45.
+// GROUPS producer groups of four warps, one k-block in flight each in registers
+// (32 KB of loads), plus one MMA warp. Two groups leave half of the SM's registers
+// to a second CTA or to the lidar of another rollout chain or stream (64 KB in
+// flight an SM, 128 KB with two CTAs); four are for batches of few CTAs, whose
+// own latency counts (launch_mlp_fwd). Shared memory is kept to 54 KB either way,
+// two stages that the groups fill in turn: the SM's L1 is what its resident CTAs
+// leave of 256 KB, and that other lidar gathers its cells through it
+// (k_lidar_track at 4096 cars x 1081 beams takes 119 us with 224 KB of L1, 122
+// with 118 KB, 133 with 28 KB). So W1 takes the place of W0's stages once layer 1
+// is done (a bulk copy behind the first tanh), and a group keeps its k-block in
+// registers until a stage is free: with a stage a group (102 KB) the four took
+// 18.7 us at 2048 samples x 1086 inputs against 17.6, two groups 20.3. The
+// TMA-staged kernel below (200 KB) in this place made a 64-step rollout of 4096
+// cars in 16 chains 7.12 ms against 6.45.
+constexpr int FWD_STAGES = 2;
 template <int GROUPS>
 struct FwdCfg {
   static constexpr int THREADS = (GROUPS * 4 + 1) * 32;
   static constexpr int MMA_WARP = GROUPS * 4;
   static constexpr int OFF_A = 0;  // GROUPS x A; H = [h | 1 | 0] reuses A[0], A[1]
-  static constexpr int OFF_B = OFF_A + GROUPS * A_BYTES;
+  static constexpr int OFF_B = OFF_A + FWD_STAGES * A_BYTES;
   static constexpr int OFF_W1 = OFF_B;  // takes the place of W0's stages once layer 1 is done
-  static constexpr int OFF_W2 = OFF_B + GROUPS * B_BYTES;
+  static constexpr int OFF_W2 = OFF_B + FWD_STAGES * B_BYTES;
   static constexpr int OFF_BAR = OFF_W2 + 2 * 16 * 128;
   static constexpr int SMEM_BYTES = OFF_BAR + 128 + 1024;  // + barriers, + alignment slack
-  static_assert((2 * GROUPS + 4) * 8 + 8 <= 128, "barriers, the TMEM slot and the abort word fit their 128 bytes");
+  static_assert((FWD_STAGES + GROUPS + 4) * 8 + 8 <= 128, "barriers, the TMEM slot and the abort word fit their 128 bytes");
 };
 
 
-// Grid: one CTA per 128 samples. Warps 0-7 form two producer groups; group
-// g loads k-blocks g, g+2, g+4, ... of X (thread = sample row) and of W0 into
-// stage g, then arrives on full[g]. Warp 8 waits on full[kb % 2], issues the
-// four K=16 MMAs of the block and commits to empty[kb % 2]; after the last
-// block it commits to `done`. Warps 0-3 (TMEM lanes 0-127) then run the
-// epilogues and issue layers 2 and 3.
+// Grid: one CTA per 128 samples. Group g (warps 4 g to 4 g + 3) loads k-blocks
+// g, g + GROUPS, ... of X (thread = sample row) and of W0, writes k-block kb into
+// stage kb % FWD_STAGES once the one before it there is consumed (empty[g], a
+// barrier per group: a group may come back to a stage that another has used
+// since) and arrives on the stage's full. The MMA warp waits on it, issues the
+// four K=16 MMAs of the block and commits to the empty of the group that writes
+// the stage next; after the last block it commits to `done`. Warps 0-7 then run
+// the epilogues, two threads a sample (TMEM lanes 0-127), and thread 0 issues
+// layers 2 and 3.
 template <int GROUPS>
 __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
     k_mlp_fwd(const float* x, int in, int cols, int c0, int c1, const uint4* w0s, int kblocks, const uint4* w1s,
@@ -72,7 +79,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
   const uint32_t raw = tc::smem_u32(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint64_t* empty = full + GROUPS;
+  uint64_t* empty = full + FWD_STAGES;
   uint64_t* done = empty + GROUPS;
   uint64_t* drain = done + 1;  // [2]: thread 0's and the MMA lane's final commits after a timeout
   uint64_t* w1bar = drain + 2;
@@ -86,10 +93,8 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
   const bool live = c < c1;
 
   if (tid == 0) {
-    for (int g = 0; g < GROUPS; ++g) {
-      tc::mbar_init(&full[g], TILE);
-      tc::mbar_init(&empty[g], 1);
-    }
+    for (int st = 0; st < FWD_STAGES; ++st) tc::mbar_init(&full[st], TILE);
+    for (int g = 0; g < GROUPS; ++g) tc::mbar_init(&empty[g], 1);
     tc::mbar_init(done, 1);
     tc::mbar_init(w1bar, 1);
     tc::mbar_init(&drain[0], 1);
@@ -117,9 +122,9 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
 
   if (warp < MMA_WARP) {
     // ---- producers: layer-1 operands, one k-block per group in flight ----
-    const int g = warp >> 2;
-    uint8_t* A = smem + OFF_A + g * A_BYTES;
-    uint4* B = reinterpret_cast<uint4*>(smem + OFF_B + g * B_BYTES);
+    const int g = warp >> 2, st = g % FWD_STAGES;  // GROUPS is a multiple of the stages
+    uint8_t* A = smem + OFF_A + st * A_BYTES;
+    uint4* B = reinterpret_cast<uint4*>(smem + OFF_B + st * B_BYTES);
     for (int j = 0;; ++j) {
       const int kb = g + GROUPS * j;
       if (kb >= kblocks) break;
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
       const uint4* src = w0s + (long)kb * (B_BYTES / 16);
 #pragma unroll
       for (int e = 0; e < 4; ++e) wb[e] = __ldcg(src + r + e * TILE);
-      if (j >= 1 && !tc::mbar_wait_abort(&empty[g], (j - 1) & 1, abort, limit)) ok = false;
+      if (kb >= FWD_STAGES && !tc::mbar_wait_abort(&empty[g], ((kb - FWD_STAGES) / GROUPS) & 1, abort, limit)) ok = false;
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         uint4 pk = make_uint4(tc::pack_bf16(v[8 * q], v[8 * q + 1]), tc::pack_bf16(v[8 * q + 2], v[8 * q + 3]),
@@ -143,21 +148,21 @@ __global__ void __launch_bounds__(FwdCfg<GROUPS>::THREADS, GROUPS == 2 ? 2 : 1)
 #pragma unroll
       for (int e = 0; e < 4; ++e) B[r + e * TILE] = wb[e];
       tc::fence_proxy_async_smem();
-      tc::mbar_arrive(&full[g]);
+      tc::mbar_arrive(&full[st]);
     }
   } else if ((tid & 31) == 0) {
     // ---- MMA issuer: layer 1 ----
     for (int kb = 0; kb < kblocks; ++kb) {
-      const int g = kb % GROUPS;
-      if (!tc::mbar_wait_abort(&full[g], (kb / GROUPS) & 1, abort, limit)) ok = false;
+      const int st = kb % FWD_STAGES;
+      if (!tc::mbar_wait_abort(&full[st], (kb / FWD_STAGES) & 1, abort, limit)) ok = false;
       if (*abort) continue;  // issue nothing after a timeout
       issued = true;
       tc::tc_fence_after();
-      const uint64_t ad = tc::sdesc_sw128(tc::smem_u32(smem + OFF_A + g * A_BYTES));
-      const uint64_t bd = tc::sdesc_sw128(tc::smem_u32(smem + OFF_B + g * B_BYTES));
+      const uint64_t ad = tc::sdesc_sw128(tc::smem_u32(smem + OFF_A + st * A_BYTES));
+      const uint64_t bd = tc::sdesc_sw128(tc::smem_u32(smem + OFF_B + st * B_BYTES));
 #pragma unroll
       for (int k = 0; k < 4; ++k) tc::mma_bf16(tmem, ad + 2 * k, bd + 2 * k, id64, (kb | k) ? 1u : 0u);
-      tc::mma_commit(&empty[g]);
+      tc::mma_commit(&empty[(kb + FWD_STAGES) % GROUPS]);  // the group that writes this stage next
     }
     if (!*abort) tc::mma_commit(done);
   }
@@ -474,8 +479,8 @@ cudaError_t launch_mlp_fwd(const float* x, int in, int cols, const uint8_t* pack
   // Wide inputs with more 128-sample tiles than SMs and 16-byte aligned sample columns: one
   // persistent CTA per SM, each running ahead into its next tile (65536 cars, 1086 inputs: 72 us;
   // without that alignment 40001 cars took 60 us in the register-staged kernel). With no more
-  // tiles than SMs a CTA has one tile; its TMA-staged form is the faster by itself (4096 cars: 18 us
-  // against 22), but the small kernel leaves the SM its L1 (FwdCfg).
+  // tiles than SMs a CTA has one tile, and the small kernel is no slower (4096 cars: 17.6 us both)
+  // and leaves the SM its L1 (FwdCfg).
   CUtensorMap xmap;
   if (kb > 4 && sms > 0 && tiles > sms && (cols & 3) == 0 && (c0 & 3) == 0 &&
       (reinterpret_cast<uintptr_t>(x) & 15) == 0 &&
@@ -488,10 +493,16 @@ cudaError_t launch_mlp_fwd(const float* x, int in, int cols, const uint8_t* pack
     return launch_early_if(c1 - c0 == cols, k_mlp_fwd_tma, dim3(sms), TmaCfg::THREADS, TmaCfg::SMEM_BYTES, st, xmap,
                            cols, c0, c1, w0, kb, w1, w2, h1, h2, o, write_hidden, sa, err);
   }
-  // Few tiles in the whole batch (of which [c0, c1) may be one chain's part): four k-blocks in
-  // flight (22 samples x 455 inputs: 14.4 us; two cost 0.8 us more). More tiles share
-  // their SMs with a lidar and leave it the L1.
-  if (kb > 2 && (cols + TILE - 1) / TILE <= 8)
+  // Four k-blocks in flight where a CTA's own latency counts: in batches of at most 8 tiles (of
+  // which [c0, c1) may be one chain's part; 24 samples x 460 inputs: 10.9 us against 11.6), and for
+  // more than 10 k-blocks in whole batches of at most a tile for every other SM. There a step of 4096
+  // cars x 1081 beams alone on the GPU takes 140 us against 153 with two, one of a single-chain
+  // rollout of 2048 cars 101 against 113, a PPO rollout of 2048 cars x 32 steps 2.61 ms against 3.00;
+  // among steps of other sims, whose lidars such CTAs keep off their SMs, 96.9 us against 95.2. The
+  // fewer the k-blocks, the more that weighs (4096 cars x 540 beams among others 59.3 us against 57.7,
+  // alone 99 against 105; 2999 x 271 among others 32.5 against 30.5), as with more tiles (forward and
+  // backward of 1086 inputs among others: 9728 samples 55.8 us against 58.5, 16384 75.3 against 69.2).
+  if (kb > 2 && ((cols + TILE - 1) / TILE <= 8 || (kb > 10 && c1 - c0 == cols && 2 * tiles <= sms)))
     return fwd_launch<4>(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
   return fwd_launch<2>(x, in, cols, c0, c1, kb, w0, w1, w2, h1, h2, o, write_hidden, sa, err, st);
 }
