@@ -161,24 +161,15 @@ __device__ __forceinline__ void load_bias(const float* bias, int n, int N, float
   }
 }
 
-// A thread's loss sums over its tiles: FP32 within 16 columns, beyond that FP32 with the rounding errors carried
-// (Knuth's two-sum; FP64 additions are slow here), added to sums[0], sums[1] once per warp in FP64.
+// A thread's loss sums over its tiles: FP32 within 16 columns, FP64 beyond, added to sums[0], sums[1] once per warp.
 struct LossSums {
-  float s[2] = {0.0f, 0.0f}, c[2] = {0.0f, 0.0f};
+  double s[2] = {0.0, 0.0};
   double* sums;
-  __device__ __forceinline__ void add(float se, float ae) {
-    const float x[2] = {se, ae};
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const float t = s[k] + x[k], b = t - s[k];
-      c[k] += (s[k] - (t - b)) + (x[k] - b);
-      s[k] = t;
-    }
-  }
+  __device__ __forceinline__ void add(float se, float ae) { s[0] += (double)se, s[1] += (double)ae; }
   __device__ __forceinline__ void flush() {
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-      double d = (double)s[k] + (double)c[k];
+      double d = s[k];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
       if ((threadIdx.x & 31) == 0) atomicAdd(sums + k, d);
