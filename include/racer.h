@@ -331,7 +331,8 @@ int racer_surrogate_bind(racer_surrogate* surrogate, racer_sim* sim);
 int racer_surrogate_set_fused(racer_surrogate* surrogate, int fused);
 /* Keep the training set's exact labels after their first tracing (enable = 1,
  * the default; FP32, built by racer_surrogate_set_poses when the set's labels
- * fit in 32 GB) so later epochs copy instead of tracing again: the same bits.
+ * fit in 32 GB) so later epochs read them in place instead of tracing again:
+ * the same bits.
  * enable = 0 traces every batch every time (and frees the cache). */
 int racer_surrogate_set_label_cache(racer_surrogate* surrogate, int enable);
 /* Held-out error on `batches` fresh batches drawn with `seed`, surrogate vs exact. */

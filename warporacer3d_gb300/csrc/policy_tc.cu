@@ -159,9 +159,10 @@ __global__ void __launch_bounds__(128, 4)
 }
 
 // grad[n * ldg + m] = sum_z P[z][m][n] for m < mreal, n < nreal (the GEMM row
-// m is the weight's input index, column n its output row). One warp per
-// element: lane l sums the partials z = l, l + 32, ... in order, then a fixed
-// shuffle tree adds the lanes (deterministic).
+// m is the weight's input index, column n its output row). A block has 32
+// elements, a lane each, and 32 warps: warp w sums the partials z = w, w + 32,
+// ... in order (reads of 128 bytes), the sums are turned over in shared memory
+// and a fixed shuffle tree adds the 32 of an element (deterministic).
 constexpr int RED_ELEMENTS = 32;
 __global__ void __launch_bounds__(RED_ELEMENTS * 32) k_wgrad_reduce(const float* __restrict__ P, int splits, int mrows,
                                                                     int nreal, int mreal, float* grad, int ldg) {

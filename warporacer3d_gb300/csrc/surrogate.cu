@@ -50,7 +50,7 @@
 // layer with uniform heading; their labels come from the exact tracer
 // (k_pose_frames + k_lidar) batch by batch. Training walks the pose set in
 // order, epoch after epoch, so each batch's labels are kept after their first
-// tracing (label cache, FP32, up to 32 GB) and copied back in later epochs: the
+// tracing (label cache, FP32, up to 32 GB) and read in place in later epochs: the
 // same bits without tracing the same poses again.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
