@@ -124,6 +124,11 @@ def peaks():
     return 6800.0, "fallback"
 
 
+def lidar_kernel(shape):
+    """The kernel that a one-track sim's lidar runs under `shape` (Sim.lidar_shape, Sim.autotune)."""
+    return "k_lidar_dynamic" if shape["dynamic"] else "k_lidar_flat" if shape["flat"] else "k_lidar_track"
+
+
 def dram_traffic_per_launch():
     """Per-launch DRAM bytes of the lidar kernel from the committed ncu summary, if any."""
     p = ROOT / "profiles" / "lidar_traffic.txt"
@@ -653,7 +658,7 @@ def main():
     peak, peak_kind = peaks()
     traffic = dram_traffic_per_launch()
     gather_gbs = W.gather_peak(GATHER_PEAK_BYTES, 20)
-    roofline = {"kernel": "k_lidar_track", "bound": "l2-gather", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roofline = {"kernel": lidar_kernel(lidar_shape), "bound": "l2-gather", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind, "peak_kind": "HBM copy (MEASURED_PEAKS.json)",
                 "traffic": traffic, "algorithmic_bytes_per_launch": alg_bytes, "launch_ms": lidar_ms,
                 "physics_launch_ms": phys_ms, "probes_per_beam": probes / (CARS * BEAMS),
