@@ -98,9 +98,10 @@ int racer_sim_get_lidar_shape(racer_sim* sim, racer_lidar_shape* shape);
 /* Autotuner: times `reps` lidar passes on the sim's current lidar frames for
  * every cars_per_block, wide, dynamic, flat and (with several segments)
  * split, with the segments in index order and heaviest-first (by probe
- * iterations counted in one pass), in two rounds over all shapes; keeps the
+ * iterations counted in one pass), in five rounds over all shapes; keeps the
  * shape with the fastest round and returns it with that round's mean time in
- * ms. The lidar only rewrites obs rows from the frames: the sim's state is
+ * ms (of one-track shapes within a per cent of it, one whose flat is what the
+ * rule for untuned sims takes). The lidar only rewrites obs rows from the frames: the sim's state is
  * unchanged. */
 int racer_sim_autotune(racer_sim* sim, int reps, racer_lidar_shape* best, float* best_ms);
 /* Rollout graphs (racer_rollout) as `chains` (1..16) independent chains of
