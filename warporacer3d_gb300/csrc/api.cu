@@ -1463,12 +1463,17 @@ static LidarShape from_api(const racer_lidar_shape& in) {
   return shape;
 }
 
+// What `flat` comes to for this sim.
+static bool takes_flat(const racer_sim* s, const LidarShape& shape) {
+  return s->seg.count == 1 && !shape.dynamic ? lidar_flat(shape, s->n, s->beams) : shape.flat == 1;
+}
+
 static void to_api(const racer_sim* s, const LidarShape& shape, racer_lidar_shape* out) {
   out->cars_per_block = shape.cars;
   out->wide = shape.wide;
   out->split = shape.split;
   out->dynamic = shape.dynamic;
-  out->flat = s->seg.count == 1 && !shape.dynamic ? lidar_flat(shape, s->n, s->beams) : shape.flat == 1;
+  out->flat = takes_flat(s, shape);
   int order[MAX_SEGMENTS];
   segment_order(s, shape, order);
   for (int j = 0; j < MAX_SEGMENTS; ++j) out->order[j] = j < s->seg.count ? order[j] : -1;
@@ -1478,8 +1483,8 @@ static bool same_shape(const racer_sim* s, const LidarShape& a, const LidarShape
   int oa[MAX_SEGMENTS], ob[MAX_SEGMENTS];
   segment_order(s, a, oa);
   segment_order(s, b, ob);
-  return a.cars == b.cars && a.wide == b.wide && a.split == b.split && a.dynamic == b.dynamic && a.flat == b.flat &&
-         std::equal(oa, oa + s->seg.count, ob);
+  return a.cars == b.cars && a.wide == b.wide && a.split == b.split && a.dynamic == b.dynamic &&
+         takes_flat(s, a) == takes_flat(s, b) && std::equal(oa, oa + s->seg.count, ob);
 }
 
 int racer_sim_set_chains(racer_sim* s, int chains) {
