@@ -130,6 +130,7 @@ int racer_alloc(size_t bytes, void** dev) {
   RACER_ARG(dev, "racer_alloc: null output");
   RACER_TRY(cudaMalloc(dev, bytes ? bytes : 1));
   RACER_TRY(cudaMemset(*dev, 0, bytes ? bytes : 1));
+  RACER_TRY(fills_done());
   return 0;
 }
 int racer_free(void* dev) {
@@ -1126,6 +1127,7 @@ int racer_runner_evaluate(racer_sim* s, racer_policy* p, racer_acts* a, float* s
     if ((rc = dalloc(&s->eval_reward, s->n)) || (rc = dalloc(&s->eval_crash, s->n)) ||
         (rc = dalloc(&s->eval_total, 2)))
       return rc;
+    RACER_TRY(fills_done());
   }
   RACER_TRY(cudaMemsetAsync(s->eval_reward, 0, (size_t)s->n * sizeof(double), st));
   RACER_TRY(cudaMemsetAsync(s->eval_crash, 0, (size_t)s->n * sizeof(int), st));
@@ -1183,8 +1185,10 @@ __global__ void k_pack_snapshot(const float* state, const float* obs, const floa
 int racer_sim_snapshot(racer_sim* s, float* host, int synchronize) {
   RACER_ARG(s && host, "racer_sim_snapshot: null argument");
   const size_t count = (size_t)(STATE + s->in_rows + 4) * s->n;
-  if (!s->snapshot)
+  if (!s->snapshot) {
     if (int rc = dalloc(&s->snapshot, count)) return rc;
+    RACER_TRY(fills_done());
+  }
   k_pack_snapshot<<<4 * s->sms, 256, 0, s->st>>>(s->state, s->obs, s->actions, s->reward, s->done, s->n,
                                                   s->in_rows, s->snapshot);
   RACER_LAUNCHED();

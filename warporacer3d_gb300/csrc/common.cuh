@@ -94,6 +94,11 @@ struct LidarShape {
   int sms = 152;
 };
 
+// Waits for the fills of new memory: cudaMemset runs on the legacy default stream, which a caller's non-blocking stream
+// does not wait for, so a fill queued behind other default-stream work could come after the first kernels that write the
+// memory.
+inline cudaError_t fills_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 // The current device's SM count, queried once per device (grid sizes of
 // persistent and grid-stride kernels).
 inline int device_sms() {

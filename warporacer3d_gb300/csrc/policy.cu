@@ -43,6 +43,7 @@ int policy_new(int in_rows, void* stream, racer_policy** out) {
   RACER_TRY(cudaMalloc((void**)&p->pack, mlp_pack_bytes(in_rows)));
   RACER_TRY(cudaMalloc((void**)&p->err, sizeof(int)));
   RACER_TRY(cudaMemset(p->err, 0, sizeof(int)));
+  RACER_TRY(fills_done());
   *out = p;
   return 0;
 }
@@ -114,7 +115,10 @@ int policy_forward(racer_policy* p, const float* x, int cols, float* h1, float* 
 int policy_status(racer_policy* p, int* code) {
   RACER_TRY(cudaStreamSynchronize(p->st));
   RACER_TRY(cudaMemcpy(code, p->err, sizeof(int), cudaMemcpyDeviceToHost));
-  if (*code) RACER_TRY(cudaMemset(p->err, 0, sizeof(int)));  // read and clear
+  if (*code) {  // read and clear
+    RACER_TRY(cudaMemset(p->err, 0, sizeof(int)));
+    RACER_TRY(fills_done());
+  }
   return 0;
 }
 

@@ -216,6 +216,11 @@ int backward_work_new(int in, int cols, BackwardWork** out) {
     backward_work_delete(w);
     return rc;
   }
+  if (cudaError_t e = fills_done(); e != cudaSuccess) {
+    racer_host::set_error(std::string("policy backward workspace: ") + cudaGetErrorString(e));
+    backward_work_delete(w);
+    return 2;
+  }
   if ((rc = make_tmap_bf16(&w->txb, w->xb, in, ld, ld, 128)) || (rc = make_tmap_bf16(&w->th1b, w->h1b, HA, ld, ld, 128)) ||
       (rc = make_tmap_bf16(&w->th2b, w->h2b, HA, ld, ld, 128)) || (rc = make_tmap_bf16(&w->td2f, w->d2f, H, ld, ld, 64)) ||
       (rc = make_tmap_bf16(&w->td3f, w->d3f, 16, ld, ld, 16)) || (rc = make_tmap_bf16(&w->td1f, w->d1f, H, ld, ld, 64))) {

@@ -1251,6 +1251,7 @@ int racer_surrogate_set_poses(racer_surrogate* s, long count, uint64_t seed) {
   s->lcache = nullptr;
   s->lcached.assign(0, 0);
   if (int rc = salloc(&s->poses, (size_t)count)) return rc;
+  RACER_TRY(fills_done());
   s->npose = (int)count;
   const size_t cache_bytes = (size_t)count * s->L.beams * sizeof(float);
   if (s->use_cache && cache_bytes <= (32ull << 30)) {  // else trace every batch every epoch
@@ -1544,6 +1545,7 @@ int surrogate_prepare(racer_surrogate* s, racer_sim* sim) {
     return rc;
   if (!s->rsums && ((rc = salloc(&s->rsums, 2)) || (rc = salloc(&s->rmax, 1)) || (rc = salloc(&s->rcount, 2))))
     return rc;
+  RACER_TRY(fills_done());
   return 0;
 }
 
